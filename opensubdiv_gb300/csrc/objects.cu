@@ -7,6 +7,7 @@
 #include "sell.h"
 #include "stencils_batch.h"
 #include "tables.h"
+#include "units.h"
 
 #include <algorithm>
 #include <new>
@@ -102,9 +103,27 @@ struct GB300StencilTable {
     // Sliced evaluation layout (sell.h): sz, sliceSlot, idx, w x 6, outRow
     gb300::SellTable sell;
     void *sbuf[10] = {nullptr};
+    // Unit layout (units.h) of a large table with one weight array: slice, blob
+    gb300::UnitTable unit;
+    void *ubuf[2] = {nullptr};
+    int build_layouts(const void *const *b, cudaStream_t s, const char *who) {
+        const int *sizes = (const int *)b[0], *offsets = (const int *)b[1];
+        const int *indices = (const int *)b[2];
+        const int r = gb300::build_sell(numStencils, sizes, offsets, indices,
+                                        (const float *const *)b + 3, s, sell, sbuf, who);
+        if (r != GB300_OK) return r == GB300_ERR_UNSUPPORTED ? GB300_OK : r;
+        bool one = b[3] && numStencils >= gb300::kUnitTable;
+        for (int k = 4; k < 9; ++k) one = one && !b[k];
+        if (!one) return GB300_OK;
+        const int u = gb300::build_units(numStencils, sizes, offsets, indices,
+                                         (const float *)b[3], s, unit, ubuf, who);
+        if (u == GB300_ERR_OUT_OF_MEMORY) cudaGetLastError();  // the table does without
+        return u == GB300_ERR_CUDA ? u : GB300_OK;
+    }
     ~GB300StencilTable() {
         for (auto &p : buf) release(p);
         for (auto &p : sbuf) release(p);
+        for (auto &p : ubuf) release(p);
     }
 };
 
@@ -212,10 +231,7 @@ GB300StencilTable *GB300StencilTableCreate(int numStencils, int64_t nnz, const i
             return nullptr;
         }
     }
-    const int r = gb300::build_sell(numStencils, (const int *)t->buf[0], (const int *)t->buf[1],
-                                    (const int *)t->buf[2], (const float *const *)(t->buf + 3), s,
-                                    t->sell, t->sbuf, "GB300StencilTableCreate");
-    if (r != GB300_OK && r != GB300_ERR_UNSUPPORTED) {
+    if (t->build_layouts(t->buf, s, "GB300StencilTableCreate") != GB300_OK) {
         delete t;
         return nullptr;
     }
@@ -246,6 +262,7 @@ int stencil_table_num_control(const GB300StencilTable *t) { return t ? t->numCon
 }  // namespace batch
 
 const SellTable *stencil_table_sell(const GB300StencilTable *t) { return t ? &t->sell : nullptr; }
+const UnitTable *stencil_table_units(const GB300StencilTable *t) { return t ? &t->unit : nullptr; }
 
 GB300StencilTable *adopt_stencil_table(int numStencils, int64_t nnz, int numControl,
                                        void *const buf[9], cudaStream_t s, const char *who) {
@@ -257,10 +274,7 @@ GB300StencilTable *adopt_stencil_table(int numStencils, int64_t nnz, int numCont
     t->numStencils = numStencils;
     t->nnz = nnz;
     t->numControl = numControl;
-    const int r = build_sell(numStencils, (const int *)buf[0], (const int *)buf[1],
-                             (const int *)buf[2], (const float *const *)buf + 3, s, t->sell,
-                             t->sbuf, who);
-    if (r != GB300_OK && r != GB300_ERR_UNSUPPORTED) {
+    if (t->build_layouts(buf, s, who) != GB300_OK) {
         delete t;  // buffers not yet owned
         return nullptr;
     }
@@ -338,6 +352,9 @@ int table_eval(const GB300StencilTable *t, const float *src, float *const *dIn, 
                         "weights",
                         k);
     }
+    if (t->unit.numSlices > 0 && d[0] && src && units_take(src, srcStride, d[0], st[0]))
+        return eval_stencils_units(t->unit, src, d[0], st[0], length, srcStride, s,
+                                   "GB300StencilTableEval");
     if (t->sell.numSlices > 0 && t->sell.idx) {
         const float *sw[6];
         for (int k = 0; k < 6; ++k) sw[k] = d[k] ? t->sell.w[k] : nullptr;

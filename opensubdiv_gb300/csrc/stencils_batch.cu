@@ -19,6 +19,7 @@
 #include "stencil_eval.cuh"
 #include "stencils_batch.h"
 #include "tables.h"
+#include "unit_ring.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -167,6 +168,7 @@ __device__ __forceinline__ void tile_threads12(const Job &j, const Meta &m, cons
 // wide over 16-byte aligned rows (one 12-column pass), at most 4 floats over 16-byte aligned
 // rows (one 4-column pass; sliced batches only).
 constexpr int kAny = 0, kWide = 1, kNarrow = 2;
+constexpr int kUnits = 3;  // every job reads its table's unit layout (mode 3)
 
 // One slice of a sliced job by one warp (lane = stencil): entry j of the 32 stencils at a time,
 // index and weight from the stage (slot base `slot0`) or, for a slice wider than the stage,
@@ -454,6 +456,68 @@ __global__ void __launch_bounds__(kThreads, (Ring<CLS, SLICED>::kMinBlocks))
     }
 }
 
+// Unit jobs: the slices of every job's unit layout (units.h), one list over all of them, as the
+// table kernel (stencils_units.cu) takes those of one table.
+__global__ void __launch_bounds__(units::kThreads, 1) k_stencils_batch_units(const Args a) {
+    using namespace units;
+    extern __shared__ __align__(128) char smem[];
+    __shared__ Queue queue[units::kWarps];
+    __shared__ int slotJob[units::kWarps][kAhead];
+    __shared__ int claimed;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) claimed = 0;
+    queue_init(queue);
+    const int count = (a.numTiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
+    Queue &q = queue[warp];
+    char *bytes = smem + (size_t)warp * kWarpBytes;
+    const uint64_t pol_stream = l2_evict_first();
+    int4 d = make_int4(0, 0, 0, 0);
+    int jc = 0;  // job of the claimed slice (claims only grow)
+    bool more = true;
+    auto claim = [&]() {
+        int k = 0;
+        if (lane == 0) k = atomicAdd(&claimed, 1);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        more = k < count;
+        if (!more) return;
+        const int t = (int)blockIdx.x + k * (int)gridDim.x;
+        for (;;) {  // the last job whose first slice is <= t
+            const int n = jc + 1 + lane;
+            const int pass = __popc(__ballot_sync(0xffffffffu, n < a.numJobs &&
+                                                                   __ldg(a.tileBase + n) <= t));
+            jc += pass;
+            if (pass < 32) break;
+        }
+        d = __ldg(reinterpret_cast<const int4 *>(a.jobs[jc].slSz) +
+                  (t - __ldg(a.tileBase + jc)));
+    };
+    claim();
+    Feed f;
+    Far far{reinterpret_cast<float4 *>(bytes + (size_t)kUnitRing * 128), q.far};
+    for (;; ++f.popped) {
+        while (more && f.room(q, d.w)) {
+            if (lane == 0) slotJob[warp][f.pushed % kAhead] = jc;
+            f.push(q, bytes, reinterpret_cast<const char *>(a.jobs[jc].slIdx), d, lane,
+                   pol_stream);
+            claim();
+        }
+        if (f.popped == f.pushed) return;
+        const int s = f.popped % kAhead;
+        if (!ring::wait(&q.full[s], (uint32_t)(f.popped / kAhead) & 1, a.status)) return;
+        const Job &j = a.jobs[slotJob[warp][s]];
+        struct View {
+            const float *src;
+            float *dst[1];
+            int dstStride[1], srcStride, length;
+        };
+        const View v{j.src, {j.dst[0]}, {j.dstStride[0]}, j.srcStride, j.length};
+        if (!consume(v, q, bytes, reinterpret_cast<const char *>(j.slIdx), far, s, lane,
+                     unit_shift(v.length), pol_stream, a.status))
+            return;
+        __syncwarp();
+    }
+}
+
 // Row i of a pad job: 4, 8, 12 or 16 floats, 128-bit stores.
 __device__ __forceinline__ void pad_row(const PadJob &j, long long i) {
     const float *row = j.src + i * j.srcStride;
@@ -551,6 +615,10 @@ int plan_tiles(Job *jobs, const double *meanSize, int n, int tileStencils, int w
     for (int k = 0; k < n; ++k) {
         Job &j = jobs[k];
         tileBase[k] = (int)total;
+        if (j.mode == 3) {  // a tile is a slice of units
+            total += j.numSlices;
+            continue;
+        }
         if (j.slSz) {
             j.mode = 2;
             j.tileStencils = kSliceTile * 32;
@@ -568,15 +636,15 @@ int plan_tiles(Job *jobs, const double *meanSize, int n, int tileStencils, int w
 int set_smem_attribute() {
     static std::atomic<uint64_t> attr{0};  // devices whose function attribute is set
     return once_per_device(attr, [] {
-        void (*const kernels[5])(Args) = {
+        void (*const kernels[6])(Args) = {
             k_stencils_batch<kAny, false>, k_stencils_batch<kWide, false>,
             k_stencils_batch<kAny, true>, k_stencils_batch<kWide, true>,
-            k_stencils_batch<kNarrow, true>};
-        const size_t bytes[5] = {Ring<kAny, false>::kSmem, Ring<kWide, false>::kSmem,
+            k_stencils_batch<kNarrow, true>, k_stencils_batch_units};
+        const size_t bytes[6] = {Ring<kAny, false>::kSmem, Ring<kWide, false>::kSmem,
                                  Ring<kAny, true>::kSmem, Ring<kWide, true>::kSmem,
-                                 Ring<kNarrow, true>::kSmem};
+                                 Ring<kNarrow, true>::kSmem, units::kSmemBytes};
         int st = GB300_OK;
-        for (int k = 0; k < 5 && st == GB300_OK; ++k)
+        for (int k = 0; k < 6 && st == GB300_OK; ++k)
             st = check_cuda(cudaFuncSetAttribute(kernels[k],
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)bytes[k]),
@@ -591,6 +659,13 @@ int launch_jobs(const Job *dJobs, const int *dTileBase, int n, int numTiles, int
     int st = set_smem_attribute();
     if (st != GB300_OK) return st;
     if (numTiles == 0) return ok();
+    if (cls == kUnits) {
+        Args a{dJobs, dTileBase, n, numTiles, dCounter, dStatus, 0};
+        k_stencils_batch_units<<<std::min(numTiles, num_sms()), units::kThreads,
+                                 units::kSmemBytes, s>>>(a);
+        count_launch();
+        return check_launch("batched EvalStencils");
+    }
     if (cls == kNarrow && !sliced)
         return fail(GB300_ERR_INVALID_ARGUMENT, "batched EvalStencils: narrow class unsliced");
     if (dynamic) {
@@ -621,7 +696,7 @@ int launch_jobs(const Job *dJobs, const int *dTileBase, int n, int numTiles, int
 
 struct Config {
     int tileStencils = 256;  // stencils per tile
-    int ctasPerSm = 2;       // persistent CTAs per SM
+    int ctasPerSm = 3;       // persistent CTAs per SM, as far as the kernels' registers allow
     int warpThreshold = 64;  // mean stencil size above which a job uses warp-per-stencil
     int dynamic = 1;         // tiles claimed from a work counter (else round-robin)
 };
@@ -655,21 +730,27 @@ uint64_t work_signature(const std::vector<Job> &jobs, const std::vector<double> 
 using namespace gb300;
 using namespace gb300::batch;
 
+constexpr int kParts = 4;
+
 struct GB300StencilBatch {
     // in launch order, one launch per part: the general jobs, the jobs at most 4 floats wide
     // over 16-byte aligned rows (sliced batches: the 4-column instantiation), the jobs 9-12
-    // floats wide over 16-byte aligned rows (the 12-wide instantiation); each part largest
-    // first
+    // floats wide over 16-byte aligned rows (the 12-wide instantiation), and, of a sliced batch,
+    // the jobs that the unit layout takes; each part largest first
     std::vector<Job> jobs;
     std::vector<double> mean;  // mean stencil size per job (same order)
-    int part[3] = {0, 0, 0};   // jobs per part
+    int part[kParts] = {};     // jobs per part
     bool sliced = false;       // every job reads its table's sliced layout (mode 2)
     Config cfg;
     Job *dJobs = nullptr;      // jobs, then the tile prefixes of the parts (part[p] + 1 ints
     int *dTileBase = nullptr;  // each)
     int *dCounter = nullptr;   // [1] status word; [0], [2], [3] work counters of the parts
-    int partTiles[3] = {0, 0, 0};
-    int numTiles() const { return partTiles[0] + partTiles[1] + partTiles[2]; }
+    int partTiles[kParts] = {};
+    int numTiles() const {
+        int n = 0;
+        for (int t : partTiles) n += t;
+        return n;
+    }
     uint64_t signature = 0;
     cudaGraphExec_t graph = nullptr;  // pad copy + counter reset + kernel, on first use
     cudaStream_t capture = nullptr;
@@ -698,21 +779,21 @@ namespace {
 std::mutex g_tuneLock;
 std::map<uint64_t, Config> g_tuned;  // work signature -> best config
 
-constexpr int kPartClass[3] = {kAny, kNarrow, kWide};
-constexpr int kPartCounter[3] = {0, 3, 2};
+constexpr int kPartClass[kParts] = {kAny, kNarrow, kWide, kUnits};
+constexpr int kPartCounter[kParts] = {0, 3, 2, 0};  // the last one claims within its CTAs
 
 // Applies b->cfg: job modes, tile sizes and the tile prefixes, uploaded to the device.
 int upload_plan(GB300StencilBatch *b, cudaStream_t s) {
     const int n = (int)b->jobs.size();
-    std::vector<int> base(n + 3);
-    for (int p = 0, j0 = 0; p < 3; j0 += b->part[p], ++p)
+    std::vector<int> base(n + kParts);
+    for (int p = 0, j0 = 0; p < kParts; j0 += b->part[p], ++p)
         b->partTiles[p] = plan_tiles(b->jobs.data() + j0, b->mean.data() + j0, b->part[p],
                                      b->cfg.tileStencils, b->cfg.warpThreshold,
                                      base.data() + j0 + p);
     int st = check_cuda(cudaMemcpyAsync(b->dJobs, b->jobs.data(), n * sizeof(Job),
                                         cudaMemcpyHostToDevice, s), "batch jobs");
     if (st != GB300_OK) return st;
-    st = check_cuda(cudaMemcpyAsync(b->dTileBase, base.data(), (n + 3) * sizeof(int),
+    st = check_cuda(cudaMemcpyAsync(b->dTileBase, base.data(), (n + kParts) * sizeof(int),
                                     cudaMemcpyHostToDevice, s), "batch jobs");
     if (st != GB300_OK) return st;
     return check_cuda(cudaStreamSynchronize(s), "batch jobs");
@@ -721,7 +802,7 @@ int upload_plan(GB300StencilBatch *b, cudaStream_t s) {
 int launch_batch(GB300StencilBatch *b, cudaStream_t s) {
     int st = launch_pad(b->dPad, b->dPadBase, b->numPad, b->padRows, s);
     if (st != GB300_OK) return st;
-    for (int p = 0, j0 = 0; p < 3; j0 += b->part[p], ++p) {
+    for (int p = 0, j0 = 0; p < kParts; j0 += b->part[p], ++p) {
         st = launch_jobs(b->dJobs + j0, b->dTileBase + j0 + p, b->part[p], b->partTiles[p],
                          b->dCounter + kPartCounter[p], b->dCounter + 1, b->cfg.ctasPerSm, s,
                          b->cfg.dynamic, kPartClass[p], b->sliced);
@@ -856,7 +937,9 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
                mean[y] * jobs[y].numStencils * jobs[y].length;
     });
     std::vector<int> rows;
+    std::vector<const UnitTable *> units;
     for (int i : order) {
+        units.push_back(stencil_table_units(tables[i]));
         b->jobs.push_back(jobs[i]);
         b->mean.push_back(mean[i]);
         rows.push_back(stencil_table_num_control(tables[i]));
@@ -870,6 +953,16 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
         delete b;
         return nullptr;
     }
+    for (size_t k = 0; k < b->jobs.size(); ++k) {
+        Job &j = b->jobs[k];
+        if (!b->sliced || units[k]->numSlices == 0 ||
+            !units_take(j.src, j.srcStride, j.dst[0], j.dstStride[0]))
+            continue;
+        j.mode = 3;
+        j.slSz = reinterpret_cast<const int *>(units[k]->slice);
+        j.slIdx = reinterpret_cast<const int *>(units[k]->blob);
+        j.numSlices = units[k]->numSlices;
+    }
     // parts: jobs one output 9-12 floats wide over 16-byte aligned rows (stride >= 12) go to
     // the 12-wide launch, jobs at most 4 floats wide over 16-byte aligned rows of a sliced
     // batch to the 4-column launch, the rest to the general one (order within each part kept:
@@ -877,12 +970,13 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
     {
         const bool sliced = b->sliced;
         auto part_of = [sliced](const Job &j) {
+            if (j.mode == 3) return 3;
             if (j.vw >= 4 && j.length > 8 && j.length <= 12) return 2;
             if (sliced && j.vw >= 4 && j.length <= 4) return 1;
             return 0;
         };
-        std::vector<Job> pj[3];
-        std::vector<double> pm[3];
+        std::vector<Job> pj[kParts];
+        std::vector<double> pm[kParts];
         for (size_t k = 0; k < b->jobs.size(); ++k) {
             const int p = part_of(b->jobs[k]);
             pj[p].push_back(b->jobs[k]);
@@ -890,7 +984,7 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
         }
         b->jobs.clear();
         b->mean.clear();
-        for (int p = 0; p < 3; ++p) {
+        for (int p = 0; p < kParts; ++p) {
             b->part[p] = (int)pj[p].size();
             b->jobs.insert(b->jobs.end(), pj[p].begin(), pj[p].end());
             b->mean.insert(b->mean.end(), pm[p].begin(), pm[p].end());
@@ -914,7 +1008,7 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
         if (it != g_tuned.end()) b->cfg = it->second;
     }
     const size_t jobBytes = ((numJobs * sizeof(Job) + 255) / 256) * 256;
-    if (check_cuda(cudaMalloc((void **)&b->dJobs, jobBytes + (numJobs + 3) * sizeof(int)),
+    if (check_cuda(cudaMalloc((void **)&b->dJobs, jobBytes + (numJobs + kParts) * sizeof(int)),
                    "batch jobs") != GB300_OK) {
         b->dJobs = nullptr;
         delete b;
@@ -972,7 +1066,7 @@ int GB300StencilBatchEvalGraph(GB300StencilBatch *b, void *stream) {
     }
     int st = check_cuda(cudaGraphLaunch(b->graph, s), "GB300StencilBatchEvalGraph");
     if (st != GB300_OK) return st;
-    for (int p = 0; p < 3; ++p)
+    for (int p = 0; p < kParts; ++p)
         if (b->partTiles[p]) count_launch();
     return ok();
 }

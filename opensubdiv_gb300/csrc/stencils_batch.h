@@ -24,11 +24,12 @@ struct Job {
     const int *sizes, *offsets;
     int length, srcStride;
     int vw;             // source rows: 8 = 256-bit loads, 4 = 128-bit loads, 1 = scalar
-    int mode;           // 0: one stencil per thread, 1: one stencil per warp, 2: sliced
+    int mode;           // 0: one stencil per thread, 1: one stencil per warp, 2: sliced, 3: units
     int numStencils;
     int tileStencils;   // stencils per tile of this job
     // the table's sliced layout (sell.h), null when absent: mode 2 tiles are kSliceTile slices
-    // (one per consumer warp, one stencil per lane) read from it
+    // (one per consumer warp, one stencil per lane) read from it.  Mode 3 (units.h): slSz is the
+    // slice descriptors, slIdx the blobs, numSlices their number
     const int *slSz, *slSlot, *slIdx, *slRow;
     const float *slW;
     int numSlices;

@@ -654,9 +654,14 @@ int eval_stencils_sell(const SellTable &t, const float *src, float *const *dst,
 namespace gb300 {
 
 int status_word_address(int **out) {
+    static std::atomic<int *> cache[64];  // per device: the symbol's address does not change
+    int dev = 0;
+    const bool cached = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
+    if (cached && (*out = cache[dev].load(std::memory_order_acquire))) return GB300_OK;
     void *p = nullptr;
     const int st = check_cuda(cudaGetSymbolAddress(&p, g_status), "status word address");
     *out = (int *)p;
+    if (st == GB300_OK && cached) cache[dev].store((int *)p, std::memory_order_release);
     return st;
 }
 

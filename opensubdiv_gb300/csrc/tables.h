@@ -10,12 +10,16 @@ struct GB300StencilTable;
 namespace gb300 {
 
 struct SellTable;
+struct UnitTable;
 
 // The table's sliced evaluation layout (numSlices 0 when it has none).
 const SellTable *stencil_table_sell(const GB300StencilTable *table);
 
+// The table's unit layout (numSlices 0 when it has none).
+const UnitTable *stencil_table_units(const GB300StencilTable *table);
+
 // Wraps device buffers (sizes, offsets, indices, w, du, dv, duu, duv, dvv; unused = null, all
-// allocated with cudaMalloc) in a table object that owns them, and builds its sliced
+// allocated with cudaMalloc) in a table object that owns them, and builds its
 // evaluation layout on stream `s`.  numControl = largest control index + 1.  Returns null
 // (buffers untouched, status recorded) when out of host memory or when the layout build
 // fails.
