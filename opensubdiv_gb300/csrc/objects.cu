@@ -496,6 +496,7 @@ GB300PatchTable *GB300PatchTableCreate(int numArrays, const void *patchArrays,
     t->map.maxFace = hm.maxFace;
     t->map.maxDepth = hm.maxDepth;
     t->map.numPatches = numPatches;
+    t->map.set_arrays(numArrays, arr);
     ok();
     return t;
 }

@@ -21,6 +21,13 @@ struct PatchMapDevice {
     void *nodes = nullptr;
     void *handles = nullptr;
     int triangular = 0, minFace = 0, maxFace = -1, maxDepth = 0, numPatches = 0;
+    // as PatchMapView's; set_arrays fills them in from the table's host arrays
+    int numArrays = 0, first[kMapArrays] = {}, step[kMapArrays] = {};
+    void set_arrays(int n, const int *arrays) {
+        numArrays = n <= kMapArrays ? n : 0;
+        for (int a = 0, h = 0; a < numArrays; h += arrays[6 * a + 2], ++a)
+            first[a] = h, step[a] = arrays[6 * a + 4];
+    }
 };
 
 // Builds the quadtree of far/patchMap.cpp:89-202 from host arrays (6 ints per patch array,
