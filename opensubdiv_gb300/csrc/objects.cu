@@ -145,6 +145,7 @@ struct PatchSet {
 struct GB300PatchTable {
     int numArrays = 0, numPatches = 0;
     int quadFamily = 0;  // all arrays REGULAR / GREGORY_BASIS / QUADS
+    int numControl = 0;  // largest control index + 1 (rows of the source the table reads)
     int64_t numIndices = 0;
     void *arrays = nullptr, *indices = nullptr, *params = nullptr;
     PatchMapDevice map;
@@ -480,6 +481,11 @@ GB300PatchTable *GB300PatchTableCreate(int numArrays, const void *patchArrays,
     t->numPatches = numPatches;
     t->numIndices = numIndices;
     t->quadFamily = quad_family(numArrays, arr);
+    {
+        int mx = -1;
+        for (int64_t e = 0; e < numIndices; ++e) mx = std::max(mx, patchIndices[e]);
+        t->numControl = mx + 1;
+    }
     t->hostArrays.assign(arr, arr + 6 * (size_t)numArrays);
     const char *w = "GB300PatchTableCreate";
     if (!upload(&t->arrays, patchArrays, (size_t)numArrays * 24, s, w) ||
@@ -523,9 +529,34 @@ int GB300PatchTableEval(const GB300PatchTable *t, const float *src, float *dst, 
                         int srcStride, int dstStride, int duStride, int dvStride,
                         int duuStride, int duvStride, int dvvStride, int numPatchCoords,
                         const void *patchCoords, void *stream) {
-    if (!t) return fail(GB300_ERR_INVALID_ARGUMENT, "GB300PatchTableEval: null table");
+    const char *who = "GB300PatchTableEval";
+    if (!t) return fail(GB300_ERR_INVALID_ARGUMENT, "%s: null table", who);
     float *d[6] = {dst, du, dv, duu, duv, dvv};
     const int st[6] = {dstStride, duStride, dvStride, duuStride, duvStride, dvvStride};
+    cudaStream_t s = as_stream(stream);
+    // Loop tables are evaluated one point per thread, 13 rows each: rows of 3 floats are read from
+    // a copy padded to 4 (one load per row), as soon as there are more points than rows to copy
+    // (4 M points, 226 k rows: 298 us, and 238 + 4 us with the copy).  Catmull-Clark tables read a
+    // row with 3 lanes in one access; a padded copy costs them more than it saves (332 us, and
+    // 366 + 24 us over 5.7 M rows).  Not while the stream is captured: the copy's memory would
+    // become part of the caller's graph.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (src && length == 3 && srcStride >= 3 && !t->quadFamily &&
+        numPatchCoords >= 65536 && numPatchCoords >= t->numControl && t->numControl > 0 &&
+        cudaStreamIsCapturing(s, &capture) == cudaSuccess &&
+        capture == cudaStreamCaptureStatusNone) {
+        float *padded = nullptr;
+        if (scratch_alloc((void **)&padded, (size_t)t->numControl * 16, s, who) == GB300_OK) {
+            batch::PadJob j{src, padded, srcStride, length, t->numControl, 4, 0};
+            int r = batch::launch_pad_one(j, s);
+            if (r == GB300_OK)
+                r = eval_patches(padded, d, st, length, 4, numPatchCoords, patchCoords, t->arrays,
+                                 (const int *)t->indices, t->params, s, who, 0, 0, 1);
+            scratch_free(padded, s);
+            return r != GB300_OK ? r : check_launch(who);
+        }
+        cudaGetLastError();  // no stream-ordered memory: evaluate in place
+    }
     return eval_patches(src, d, st, length, srcStride, numPatchCoords, patchCoords, t->arrays,
                         (const int *)t->indices, t->params, as_stream(stream),
                         "GB300PatchTableEval", t->quadFamily);

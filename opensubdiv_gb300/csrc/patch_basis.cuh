@@ -51,14 +51,25 @@ struct Acc6 {
 // query that lands on the same patch: they are loaded with an evict-last L2 policy, so the
 // streams read or written once (query coords, outputs) do not push them out of L2.
 
-// Loads LC elements [e0, e0+LC) of control point `cv` (elements >= length read as 0).
-template <int LC>
+// Loads LC elements [e0, e0+LC) of control point `cv` (elements >= length read as 0).  V4: rows of
+// 3 or 4 elements whose 16 bytes are aligned (and inside the row's stride): one load per row;
+// elements >= length are whatever the row's stride holds, and are not written.
+template <int LC, bool V4>
 __device__ __forceinline__ void load_row(const float *__restrict__ src, int stride, int cv,
                                          int e0, int length, float (&x)[LC]) {
     const float *p = src + (size_t)cv * stride + e0;
     const uint64_t pol = l2_evict_last();
+    if constexpr (V4) {
+        static_assert(LC == 3 || LC == 4, "one quad per row");
+        const int4 v = ld_keep4(reinterpret_cast<const int *>(p), pol);
+        x[0] = __int_as_float(v.x);
+        x[1] = __int_as_float(v.y);
+        x[2] = __int_as_float(v.z);
+        if constexpr (LC == 4) x[3] = __int_as_float(v.w);
+    } else {
 #pragma unroll
-    for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? ld_src(p + c, pol) : 0.0f;
+        for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? ld_src(p + c, pol) : 0.0f;
+    }
 }
 
 // Local origin.  Every basis is a partition of unity: its value weights sum to 1 and every
@@ -68,14 +79,20 @@ __device__ __forceinline__ void load_row(const float *__restrict__ src, int stri
 // then scale with the patch's extent instead of the points' distance from the origin, and
 // the float rounding of the cancelling derivative sums (which carry the 2^depth and 4^depth
 // factors) shrinks by that ratio.  The value output adds xc back at the end.
-template <int LC>
+template <int LC, bool V4>
 __device__ __forceinline__ void load_row(const float *__restrict__ src, int stride, int cv,
                                          int e0, int length, float (&x)[LC],
                                          const float (&xc)[LC]) {
-    const float *p = src + (size_t)cv * stride + e0;
-    const uint64_t pol = l2_evict_last();
+    if constexpr (V4) {
+        load_row<LC, true>(src, stride, cv, e0, length, x);
 #pragma unroll
-    for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? ld_src(p + c, pol) - xc[c] : 0.0f;
+        for (int c = 0; c < LC; ++c) x[c] -= xc[c];
+    } else {
+        const float *p = src + (size_t)cv * stride + e0;
+        const uint64_t pol = l2_evict_last();
+#pragma unroll
+        for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? ld_src(p + c, pol) - xc[c] : 0.0f;
+    }
 }
 
 template <int LC>
@@ -165,7 +182,7 @@ __device__ __forceinline__ void tensor_accumulate(const float (&sp)[4], const fl
 }
 
 // REGULAR: 16 points in row-major (t rows, s columns) order.
-template <int LC>
+template <int LC, bool V4 = false>
 __device__ void eval_bspline(float s, float t, int boundary, const int *__restrict__ cvs,
                              const float *__restrict__ src, int stride, int e0, int length,
                              Acc6<LC> &acc) {
@@ -180,14 +197,28 @@ __device__ void eval_bspline(float s, float t, int boundary, const int *__restri
     int idx[16];
     load_indices<16>(cvs, idx);
     float xc[LC];  // point 5: the patch's (0,0) corner, never a phantom
-    load_row<LC>(src, stride, idx[5], e0, length, xc);
+    if constexpr (LC == 1) {  // all 16 rows in flight at a time
+        float x[16][1];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        float x[4][LC];
+        for (int j = 0; j < 16; ++j) load_row<1, false>(src, stride, idx[j], e0, length, x[j]);
+        xc[0] = x[5][0];
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-            load_row<LC>(src, stride, idx[4 * r + c], e0, length, x[c], xc);
-        tensor_accumulate<LC>(sp, sd, sdd, tp[r], td[r], tdd[r], x, acc);
+        for (int r = 0; r < 4; ++r) {
+            float y[4][1];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) y[c][0] = x[4 * r + c][0] - xc[0];
+            tensor_accumulate<1>(sp, sd, sdd, tp[r], td[r], tdd[r], y, acc);
+        }
+    } else {
+        load_row<LC, V4>(src, stride, idx[5], e0, length, xc);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            float x[4][LC];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                load_row<LC, V4>(src, stride, idx[4 * r + c], e0, length, x[c], xc);
+            tensor_accumulate<LC>(sp, sd, sdd, tp[r], td[r], tdd[r], x, acc);
+        }
     }
     add_origin<LC>(xc, acc);
 }
@@ -195,7 +226,7 @@ __device__ void eval_bspline(float s, float t, int boundary, const int *__restri
 // GREGORY_BASIS: 20 points; the Bezier grid is
 //   row 0: 0 1 7 5 | row 1: 2 (3,4) (8,9) 6 | row 2: 16 (18,19) (13,14) 12 | row 3: 15 17 11 10
 // where (a,b) is the pair of interior face points blended by G (patchBasis.h:346-378).
-template <int LC>
+template <int LC, bool V4 = false>
 __device__ void eval_gregory(float s, float t, const int *__restrict__ cvs,
                              const float *__restrict__ src, int stride, int e0, int length,
                              Acc6<LC> &acc) {
@@ -211,7 +242,7 @@ __device__ void eval_gregory(float s, float t, const int *__restrict__ cvs,
     int idx[20];
     load_indices<20>(cvs, idx);
     float xc[LC];  // point 0: the patch's (0,0) corner
-    load_row<LC>(src, stride, idx[0], e0, length, xc);
+    load_row<LC, V4>(src, stride, idx[0], e0, length, xc);
     // rows of the Bezier grid; interior entries are blended pairs
     constexpr int kGrid[4][4] = {{0, 1, 7, 5}, {2, -1, -2, 6}, {16, -4, -3, 12}, {15, 17, 11, 10}};
 #pragma unroll
@@ -221,14 +252,14 @@ __device__ void eval_gregory(float s, float t, const int *__restrict__ cvs,
         for (int c = 0; c < 4; ++c) {
             const int g = kGrid[r][c];
             if (g >= 0) {
-                load_row<LC>(src, stride, idx[g], e0, length, x[c], xc);
+                load_row<LC, V4>(src, stride, idx[g], e0, length, x[c], xc);
             } else {
                 // -1: (3,4) by g0; -2: (8,9) by g2; -3: (13,14) by g4; -4: (18,19) by g6
                 const int a = (g == -1) ? 3 : (g == -2) ? 8 : (g == -3) ? 13 : 18;
                 const float ga = (g == -1) ? g0 : (g == -2) ? g2 : (g == -3) ? g4 : g6;
                 float xa[LC], xb[LC];
-                load_row<LC>(src, stride, idx[a], e0, length, xa, xc);
-                load_row<LC>(src, stride, idx[a + 1], e0, length, xb, xc);
+                load_row<LC, V4>(src, stride, idx[a], e0, length, xa, xc);
+                load_row<LC, V4>(src, stride, idx[a + 1], e0, length, xb, xc);
 #pragma unroll
                 for (int k = 0; k < LC; ++k) x[c][k] = ga * xa[k] + (1.0f - ga) * xb[k];
             }
@@ -293,7 +324,7 @@ __device__ __forceinline__ void bezier_tri_weights(float u, float v, int ds, int
 
 // GREGORY_TRIANGLE: 18 points mapped onto the 15 quartic Bezier points; interior Bezier
 // points 6, 7 and 10 are blends of Gregory pairs (3,4), (8,9), (13,14) (patchBasis.h:1078-1106).
-template <int LC>
+template <int LC, bool V4 = false>
 __device__ void eval_gregory_tri(float s, float t, const int *__restrict__ cvs,
                                  const float *__restrict__ src, int stride, int e0, int length,
                                  Acc6<LC> &acc) {
@@ -305,20 +336,20 @@ __device__ void eval_gregory_tri(float s, float t, const int *__restrict__ cvs,
     // Bezier point m comes from Gregory point kBez[m] (or a blended pair for 6, 7, 10)
     constexpr int kBez[15] = {0, 1, 15, 7, 5, 2, -1, -2, 6, 17, -3, 16, 11, 12, 10};
     float xc[LC];  // point 0: the (0,0) corner
-    load_row<LC>(src, stride, __ldg(cvs), e0, length, xc);
+    load_row<LC, V4>(src, stride, __ldg(cvs), e0, length, xc);
     float B[15][LC];
 #pragma unroll
     for (int m = 0; m < 15; ++m) {
         const int gi = kBez[m];
         if (gi >= 0) {
-            load_row<LC>(src, stride, __ldg(cvs + gi), e0, length, B[m], xc);
+            load_row<LC, V4>(src, stride, __ldg(cvs + gi), e0, length, B[m], xc);
         } else {
             const int a = (gi == -1) ? 3 : (gi == -2) ? 8 : 13;
             const float ga = (gi == -1) ? g[0] : (gi == -2) ? g[2] : g[4];
             const float gb = (gi == -1) ? g[1] : (gi == -2) ? g[3] : g[5];
             float xa[LC], xb[LC];
-            load_row<LC>(src, stride, __ldg(cvs + a), e0, length, xa, xc);
-            load_row<LC>(src, stride, __ldg(cvs + a + 1), e0, length, xb, xc);
+            load_row<LC, V4>(src, stride, __ldg(cvs + a), e0, length, xa, xc);
+            load_row<LC, V4>(src, stride, __ldg(cvs + a + 1), e0, length, xb, xc);
 #pragma unroll
             for (int c = 0; c < LC; ++c) B[m][c] = ga * xa[c] + gb * xb[c];
         }
@@ -438,7 +469,7 @@ __device__ __forceinline__ void box_weights(int k, const float *m, float (&w)[12
     }
 }
 
-template <int LC>
+template <int LC, bool V4 = false>
 __device__ void eval_box_tri(float s, float t, int boundary, const int *__restrict__ cvs,
                              const float *__restrict__ src, int stride, int e0, int length,
                              Acc6<LC> &acc) {
@@ -454,9 +485,9 @@ __device__ void eval_box_tri(float s, float t, int boundary, const int *__restri
     {
         int idx[12];
         load_indices<12>(cvs, idx);
-        load_row<LC>(src, stride, idx[4], e0, length, xc);  // point 4: the (0,0) corner
+        load_row<LC, V4>(src, stride, idx[4], e0, length, xc);  // point 4: the (0,0) corner
 #pragma unroll
-        for (int j = 0; j < 12; ++j) load_row<LC>(src, stride, idx[j], e0, length, x[j], xc);
+        for (int j = 0; j < 12; ++j) load_row<LC, V4>(src, stride, idx[j], e0, length, x[j], xc);
     }
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -473,7 +504,7 @@ __device__ void eval_box_tri(float s, float t, int boundary, const int *__restri
     add_origin<LC>(xc, acc);
 }
 
-template <int LC>
+template <int LC, bool V4 = false>
 __device__ void eval_linear_quad(float s, float t, const int *__restrict__ cvs,
                                  const float *__restrict__ src, int stride, int e0, int length,
                                  Acc6<LC> &acc) {
@@ -483,11 +514,11 @@ __device__ void eval_linear_quad(float s, float t, const int *__restrict__ cvs,
     const float wt[4] = {-sc, -s, s, sc};
     const float wst[4] = {1.0f, -1.0f, 1.0f, -1.0f};
     float xc[LC];
-    load_row<LC>(src, stride, __ldg(cvs), e0, length, xc);
+    load_row<LC, V4>(src, stride, __ldg(cvs), e0, length, xc);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         float x[LC];
-        load_row<LC>(src, stride, __ldg(cvs + j), e0, length, x, xc);
+        load_row<LC, V4>(src, stride, __ldg(cvs + j), e0, length, x, xc);
 #pragma unroll
         for (int c = 0; c < LC; ++c) {
             acc.v[0][c] = fmaf(wp[j], x[c], acc.v[0][c]);
@@ -499,14 +530,14 @@ __device__ void eval_linear_quad(float s, float t, const int *__restrict__ cvs,
     add_origin<LC>(xc, acc);
 }
 
-template <int LC>
+template <int LC, bool V4 = false>
 __device__ void eval_linear_tri(float s, float t, const int *__restrict__ cvs,
                                 const float *__restrict__ src, int stride, int e0, int length,
                                 Acc6<LC> &acc) {
     float x0[LC], x1[LC], x2[LC];
-    load_row<LC>(src, stride, __ldg(cvs + 0), e0, length, x0);
-    load_row<LC>(src, stride, __ldg(cvs + 1), e0, length, x1, x0);
-    load_row<LC>(src, stride, __ldg(cvs + 2), e0, length, x2, x0);
+    load_row<LC, V4>(src, stride, __ldg(cvs + 0), e0, length, x0);
+    load_row<LC, V4>(src, stride, __ldg(cvs + 1), e0, length, x1, x0);
+    load_row<LC, V4>(src, stride, __ldg(cvs + 2), e0, length, x2, x0);
     // relative to point 0: P = x0 + s (x1 - x0) + t (x2 - x0)
 #pragma unroll
     for (int c = 0; c < LC; ++c) {
@@ -519,7 +550,7 @@ __device__ void eval_linear_tri(float s, float t, const int *__restrict__ cvs,
 // OsdEvaluatePatchBasis + gather for one point: normalises (s,t) into the patch, evaluates
 // the basis of `type`, accumulates into acc and returns the derivative scales d1, d2
 // (patchBasis.h:1558-1610).  Returns false for an unknown type.
-template <int LC, bool QUAD_ONLY = false>
+template <int LC, bool QUAD_ONLY = false, bool V4 = false>
 __device__ bool eval_patch_point(int type, Param p, float s, float t,
                                  const int *__restrict__ cvs, const float *__restrict__ src,
                                  int stride, int e0, int length, Acc6<LC> &acc, float &d1,
@@ -540,19 +571,19 @@ __device__ bool eval_patch_point(int type, Param p, float s, float t,
     }
     if (QUAD_ONLY) {  // Catmull-Clark tables: REGULAR, GREGORY_BASIS, QUADS
         switch (type) {
-            case 6: eval_bspline<LC>(s, t, p.boundary(), cvs, src, stride, e0, length, acc); break;
-            case 9: eval_gregory<LC>(s, t, cvs, src, stride, e0, length, acc); break;
-            case 3: eval_linear_quad<LC>(s, t, cvs, src, stride, e0, length, acc); break;
+            case 6: eval_bspline<LC, V4>(s, t, p.boundary(), cvs, src, stride, e0, length, acc); break;
+            case 9: eval_gregory<LC, V4>(s, t, cvs, src, stride, e0, length, acc); break;
+            case 3: eval_linear_quad<LC, V4>(s, t, cvs, src, stride, e0, length, acc); break;
             default: return false;
         }
     } else {
         switch (type) {
-            case 6: eval_bspline<LC>(s, t, p.boundary(), cvs, src, stride, e0, length, acc); break;
-            case 9: eval_gregory<LC>(s, t, cvs, src, stride, e0, length, acc); break;
-            case 5: eval_box_tri<LC>(s, t, p.boundary(), cvs, src, stride, e0, length, acc); break;
-            case 10: eval_gregory_tri<LC>(s, t, cvs, src, stride, e0, length, acc); break;
-            case 3: eval_linear_quad<LC>(s, t, cvs, src, stride, e0, length, acc); break;
-            case 4: eval_linear_tri<LC>(s, t, cvs, src, stride, e0, length, acc); break;
+            case 6: eval_bspline<LC, V4>(s, t, p.boundary(), cvs, src, stride, e0, length, acc); break;
+            case 9: eval_gregory<LC, V4>(s, t, cvs, src, stride, e0, length, acc); break;
+            case 5: eval_box_tri<LC, V4>(s, t, p.boundary(), cvs, src, stride, e0, length, acc); break;
+            case 10: eval_gregory_tri<LC, V4>(s, t, cvs, src, stride, e0, length, acc); break;
+            case 3: eval_linear_quad<LC, V4>(s, t, cvs, src, stride, e0, length, acc); break;
+            case 4: eval_linear_tri<LC, V4>(s, t, cvs, src, stride, e0, length, acc); break;
             default: return false;
         }
     }

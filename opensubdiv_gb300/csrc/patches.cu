@@ -50,45 +50,110 @@ struct PatchArgs {
     const Array *arrays;
     const int *indices;
     const ParamRec *params;
+    int quadRows;  // source rows are padded to quads
 };
 
 // Highest output index a derivative order needs: 0 P only, 1 P + du + dv, 2 all six.  The
 // kernels are instantiated per order so the unused accumulations compile away.
 __host__ __device__ constexpr int last_output(int order) { return order == 0 ? 0 : order == 1 ? 2 : 5; }
 
+// Elements [e0, e0 + LC) of all outputs of the point at c, and the outputs' scales.
+template <int LC, bool QUAD, bool V4>
+__device__ __forceinline__ void eval_point(const PatchArgs &a, const Coord &c, int e0,
+                                           Acc6<LC> &acc, float (&scale)[6]) {
+    acc.zero();
+    float d1 = 1.0f, d2 = 1.0f;
+    if (c.arrayIndex >= 0) {
+        const Array arr = a.arrays[c.arrayIndex];
+        const ParamRec pr = load_param(a.params + c.patchIndex);
+        const Param p{pr.field0, pr.field1};
+        const int type = p.regular() ? arr.regDesc : arr.desc;
+        const int *cvs =
+            a.indices + arr.indexBase + arr.stride * (c.patchIndex - arr.primitiveIdBase);
+        if (!eval_patch_point<LC, QUAD, V4>(type, p, c.s, c.t, cvs, a.src, a.srcStride, e0,
+                                            a.length, acc, d1, d2))
+            acc.zero();
+    }
+    scale[0] = 1.0f;
+    scale[1] = scale[2] = d1;
+    scale[3] = scale[4] = scale[5] = d2;
+}
+
+// One output of the warp's 32 points from point `first` on, whose rows
+// follow one another (stride = length = LC): written through shared memory, so that every store
+// covers whole sectors (by its thread, a row of 3 floats takes 3 stores to another
+// sector each: 29.1 M sectors written for 4 M points, where the outputs have 9.0 M).
+template <int LC>
+__device__ __forceinline__ void store_packed(float *dst, float *stage, const float (&v)[LC],
+                                             int first, int n, int lane) {
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < LC; ++m) stage[lane * LC + m] = v[m];
+    __syncwarp();
+    float *out = dst + (size_t)first * LC;
+    const int count = (n - first < 32 ? n - first : 32) * LC;
+#pragma unroll
+    for (int m = 0; m < LC; ++m)
+        if (lane + 32 * m < count) st_stream(out + lane + 32 * m, stage[lane + 32 * m]);
+}
+
 // 5 resident blocks per SM where the registers allow it without spills (0.2847 vs 0.2908 ms
 // for 4 M Loop points at LC = 3; LC = 4 would spill)
 // QUAD: Catmull-Clark tables (REGULAR / GREGORY_BASIS / QUADS only): without the Loop and
-// triangle bases the kernel fits 7 blocks per SM for orders 0 and 1 without spills.
-template <int LC, int ORDER, bool QUAD = false>
-__global__ void __launch_bounds__(128, LC == 4 ? 4 : (ORDER < 2 ? (QUAD ? 7 : 6) : 5))
+// triangle bases the kernel fits 7 blocks per SM for orders 0 and 1 without spills; it is bound by
+// instruction issue (61%), and the packed stores cost it more (79 -> 87 us for 1.7 M coords).
+// V4: source rows are read as one quad each (patch_basis.cuh).
+template <int LC, int ORDER, bool QUAD = false, bool V4 = false>
+__global__ void __launch_bounds__(128, LC == 4 ? 4 : (ORDER < 2 && !V4 ? (QUAD ? 7 : 6) : 5))
     k_eval_patches(const PatchArgs a) {
+    constexpr bool PACK = LC > 1 && (!QUAD || V4);
     const int stride = gridDim.x * blockDim.x;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.numCoords; i += stride) {
-        const Coord c = load_coord(a.coords + i);
-        for (int e0 = 0; e0 < a.length; e0 += LC) {
-            Acc6<LC> acc;
-            acc.zero();
-            float d1 = 1.0f, d2 = 1.0f;
-            if (c.arrayIndex >= 0) {
-                const Array arr = a.arrays[c.arrayIndex];
-                const ParamRec pr = load_param(a.params + c.patchIndex);
-                const Param p{pr.field0, pr.field1};
-                const int type = p.regular() ? arr.regDesc : arr.desc;
-                const int *cvs =
-                    a.indices + arr.indexBase + arr.stride * (c.patchIndex - arr.primitiveIdBase);
-                if (!eval_patch_point<LC, QUAD>(type, p, c.s, c.t, cvs, a.src, a.srcStride, e0,
-                                                a.length, acc, d1, d2))
-                    acc.zero();
+    if constexpr (!PACK) {
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.numCoords; i += stride) {
+            const Coord c = load_coord(a.coords + i);
+            for (int e0 = 0; e0 < a.length; e0 += LC) {
+                Acc6<LC> acc;
+                float scale[6];
+                eval_point<LC, QUAD, V4>(a, c, e0, acc, scale);
+#pragma unroll
+                for (int k = 0; k <= last_output(ORDER); ++k) {
+                    if (!(a.active & (1 << k))) continue;
+                    float *out = a.dst[k] + (size_t)i * a.dstStride[k] + e0;
+#pragma unroll
+                    for (int m = 0; m < LC; ++m)
+                        if (e0 + m < a.length) st_stream(out + m, acc.v[k][m] * scale[k]);
+                }
             }
-            const float scale[6] = {1.0f, d1, d1, d2, d2, d2};
+        }
+    } else {
+        // a warp's 32 points at a time, the last ones with idle lanes
+        __shared__ float stage[4][32 * LC];
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        for (int first = blockIdx.x * blockDim.x + 32 * warp; first < a.numCoords;
+             first += stride) {
+            const int i = first + lane;
+            const bool on = i < a.numCoords;
+            Coord c{-1, 0, 0, 0.0f, 0.0f};
+            if (on) c = load_coord(a.coords + i);
+            for (int e0 = 0; e0 < a.length; e0 += LC) {
+                Acc6<LC> acc;
+                float scale[6];
+                eval_point<LC, QUAD, V4>(a, c, e0, acc, scale);
 #pragma unroll
-            for (int k = 0; k <= last_output(ORDER); ++k) {
-                if (!(a.active & (1 << k))) continue;
-                float *out = a.dst[k] + (size_t)i * a.dstStride[k] + e0;
+                for (int k = 0; k <= last_output(ORDER); ++k) {
+                    if (!(a.active & (1 << k))) continue;
+                    float v[LC];
 #pragma unroll
-                for (int m = 0; m < LC; ++m)
-                    if (e0 + m < a.length) st_stream(out + m, acc.v[k][m] * scale[k]);
+                    for (int m = 0; m < LC; ++m) v[m] = acc.v[k][m] * scale[k];
+                    if (a.length == LC && a.dstStride[k] == LC) {
+                        store_packed<LC>(a.dst[k], stage[warp], v, first, a.numCoords, lane);
+                    } else if (on) {
+                        float *out = a.dst[k] + (size_t)i * a.dstStride[k] + e0;
+#pragma unroll
+                        for (int m = 0; m < LC; ++m)
+                            if (e0 + m < a.length) st_stream(out + m, v[m]);
+                    }
+                }
             }
         }
     }
@@ -155,18 +220,27 @@ void launch_lanes(int G, int grid, int threads, cudaStream_t s, const PatchArgs 
 
 template <int ORDER, bool QUAD>
 void launch_points(int length, int grid, int threads, cudaStream_t s, const PatchArgs &a) {
+    // whole quads at 16-byte aligned addresses: nothing past a row's elements is read
+    const bool v4 = ((uintptr_t)a.src & 15) == 0 && a.srcStride % 4 == 0 &&
+                    (a.length % 4 == 0 || a.quadRows);
     switch (length) {
         case 1: k_eval_patches<1, ORDER, QUAD><<<grid, threads, 0, s>>>(a); break;
         case 2: k_eval_patches<2, ORDER, QUAD><<<grid, threads, 0, s>>>(a); break;
-        case 3: k_eval_patches<3, ORDER, QUAD><<<grid, threads, 0, s>>>(a); break;
-        default: k_eval_patches<4, ORDER, QUAD><<<grid, threads, 0, s>>>(a); break;
+        case 3:
+            if (v4) k_eval_patches<3, ORDER, QUAD, true><<<grid, threads, 0, s>>>(a);
+            else k_eval_patches<3, ORDER, QUAD><<<grid, threads, 0, s>>>(a);
+            break;
+        default:
+            if (v4) k_eval_patches<4, ORDER, QUAD, true><<<grid, threads, 0, s>>>(a);
+            else k_eval_patches<4, ORDER, QUAD><<<grid, threads, 0, s>>>(a);
+            break;
     }
 }
 
 int eval_patches(const float *src, float *const *dst, const int *strides, int length,
                  int srcStride, int numCoords, const void *coords, const void *arrays,
                  const int *indices, const void *params, cudaStream_t s, const char *who,
-                 int quadFamily, int grouped) {
+                 int quadFamily, int grouped, int quadRows) {
     if (numCoords <= 0) return ok();
     if (!src || !coords || !arrays || !indices || !params)
         return fail(GB300_ERR_INVALID_ARGUMENT, "%s: null source, coord or table pointer", who);
@@ -182,6 +256,7 @@ int eval_patches(const float *src, float *const *dst, const int *strides, int le
     a.arrays = (const Array *)arrays;
     a.indices = indices;
     a.params = (const ParamRec *)params;
+    a.quadRows = quadRows;
     for (int k = 0; k < 6; ++k) {
         if (!dst[k]) continue;
         if (strides[k] < length)
@@ -242,7 +317,7 @@ int GB300EvalPatches(const float *src, float *dst, int length, int srcStride, in
     float *d[6] = {dst, 0, 0, 0, 0, 0};
     int st[6] = {dstStride, 0, 0, 0, 0, 0};
     return eval_patches(src, d, st, length, srcStride, numPatchCoords, patchCoords, patchArrays,
-                        patchIndices, patchParams, as_stream(stream), "GB300EvalPatches", 0, 0);
+                        patchIndices, patchParams, as_stream(stream), "GB300EvalPatches", 0, 0, 0);
 }
 
 int GB300EvalPatchesWithDerivatives(
@@ -254,7 +329,7 @@ int GB300EvalPatchesWithDerivatives(
     int st[6] = {dstStride, duStride, dvStride, duuStride, duvStride, dvvStride};
     return eval_patches(src, d, st, length, srcStride, numPatchCoords, patchCoords, patchArrays,
                         patchIndices, patchParams, as_stream(stream),
-                        "GB300EvalPatchesWithDerivatives", 0, 0);
+                        "GB300EvalPatchesWithDerivatives", 0, 0, 0);
 }
 
 }  // extern "C"

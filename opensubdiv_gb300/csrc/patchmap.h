@@ -53,10 +53,11 @@ int eval_stencils(const float *src, float *const *dst, const int *strides,
 // selects the element-lane kernel (known for device tables; raw-pointer calls pass 0).
 // grouped: consecutive coords mostly share a patch (a tessellation's coords), which selects
 // the one-thread-per-point kernel for every table.
+// quadRows: the source rows are a copy padded to whole quads, which may be read whole.
 int eval_patches(const float *src, float *const *dst, const int *strides, int length,
                  int srcStride, int numCoords, const void *coords, const void *arrays,
                  const int *indices, const void *params, cudaStream_t s, const char *who,
-                 int quadFamily, int grouped = 0);
+                 int quadFamily, int grouped = 0, int quadRows = 0);
 
 // Draw-time tessellation factors of every patch of a table (tess_factors.cu).
 int tess_factors(const void *arrays, int numArrays, const int *indices, const void *params,
