@@ -68,17 +68,29 @@ __device__ __forceinline__ void rates_of(const int *rateOffsets, const int *rate
     }
 }
 
+struct Totals;
+
 struct CountArgs {
     int reg, numFaces, uniformRate, fs, pq;
     const int *faceSizes, *rateOffsets, *rates;
-    int64_t *cc, *fc, *pc;  // per-face counts, [numFaces] = 0
+    Totals *counts;  // per face, [numFaces] = 0
+};
+
+// Coords, facets and ptex faces, scanned together.
+struct Totals {
+    int64_t c, f, p;
+};
+struct TotalsSum {
+    __host__ __device__ Totals operator()(const Totals &x, const Totals &y) const {
+        return Totals{x.c + y.c, x.f + y.f, x.p + y.p};
+    }
 };
 
 __global__ void __launch_bounds__(256) k_tess_count(const CountArgs a) {
     const int stride = gridDim.x * blockDim.x;
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f <= a.numFaces; f += stride) {
         if (f == a.numFaces) {
-            a.cc[f] = a.fc[f] = a.pc[f] = 0;
+            a.counts[f] = Totals{0, 0, 0};
             continue;
         }
         const int N = a.faceSizes[f];
@@ -86,9 +98,18 @@ __global__ void __launch_bounds__(256) k_tess_count(const CountArgs a) {
         rates_of(a.rateOffsets, a.rates, a.uniformRate, f, r);
         Face face;
         const bool ok = face.init(a.reg, N, r.n, r.p, a.fs, a.pq, r.one);
-        a.cc[f] = ok ? face.num_coords() : 0;
-        a.fc[f] = ok ? face.nFacets : 0;
-        a.pc[f] = N > 0 ? tess::ptex_count(a.reg, N) : 0;
+        a.counts[f] = Totals{ok ? face.num_coords() : 0, ok ? face.nFacets : 0,
+                             N > 0 ? tess::ptex_count(a.reg, N) : 0};
+    }
+}
+
+__global__ void __launch_bounds__(256) k_tess_offsets(const Totals *scan, int n, int64_t *coords,
+                                                      int64_t *facets, int64_t *ptex) {
+    for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < n; f += gridDim.x * blockDim.x) {
+        const Totals t = scan[f];
+        coords[f] = t.c;
+        facets[f] = t.f;
+        ptex[f] = t.p;
     }
 }
 
@@ -141,7 +162,7 @@ __global__ void __launch_bounds__(32) k_tess_patterns(int reg, int rate, int fs,
 // normalized (s, t) of Parameterization::ConvertCoordToNormalizedSubFace
 // (bfr/parameterization.cpp:135-162), then the PatchMap walk.
 __device__ __forceinline__ void locate_coord(const GenArgs &a, int N, int ptex0, float u, float v,
-                                             int *o) {
+                                             int *o) {  // o: 5 words
     int sub = 0;
     float s = u, t = v;
     if (N != a.reg) {
@@ -234,11 +255,11 @@ __device__ __forceinline__ int owner_of(const GenArgs &a, int f) {
     return slot < 0 ? f : a.owners[slot];
 }
 
-// One thread per face without a shared pattern: the face's coords and facets (indices already
-// offset to the mesh numbering) straight into its slice of the output.  One launch per
-// parameterization kind K present in the scheme, each generating only that kind's faces.
-template <int K>
-__global__ void __launch_bounds__(128, 8) k_tess_generate(const GenArgs a) {
+// One thread per face without a shared pattern: the face's coords or its facets (indices already
+// offset to the mesh numbering) straight into its slice of the output, for the faces of
+// parameterization kind K.
+template <int K, bool COORDS>
+__device__ __forceinline__ void generate_faces(const GenArgs &a) {
     const int stride = gridDim.x * blockDim.x;
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < a.numFaces; f += stride) {
         const int N = a.faceSizes[f];
@@ -251,16 +272,74 @@ __global__ void __launch_bounds__(128, 8) k_tess_generate(const GenArgs a) {
         const int64_t c0 = a.co[f];
         Sink o{a.coords + c0 * a.coordStride, a.coordStride, a.facets + a.fo[f] * a.facetStride,
                a.fs, a.facetStride, a.offsetIndices ? (int)c0 : 0, a.coordPairs != 0};
-        face.coords_k<K>(o);
-        face.facets_k<K>(o);
+        if constexpr (COORDS) face.coords_k<K>(o);
+        else face.facets_k<K>(o);
     }
 }
 
-// One warp per face: copies a shared pattern out (coords as float2 pairs, one lane per facet
-// with its indices offset), and locates every coord of the face on the patch table.
+// Blocks of row y of the grid generate part `first` + y.  A mesh has few distinct patterns, so the
+// launch lasts as long as one thread takes for its longest part: the parts -- two kinds of face,
+// coords and facets -- run at the same time, in one launch (41 + 23 us as a launch per kind of
+// both, and 28 us, for the per-edge rates of 69 k faces).  Each block's code is one part's.
+constexpr int kQuadParts = 0, kQsubParts = 2, kTriParts = 4;
+
+__global__ void __launch_bounds__(128, 8) k_tess_generate(const GenArgs a, int first) {
+    switch (first + (int)blockIdx.y) {
+        case kQuadParts: generate_faces<tess::kQuad, false>(a); break;
+        case kQuadParts + 1: generate_faces<tess::kQuad, true>(a); break;
+        case kQsubParts: generate_faces<tess::kQsub, false>(a); break;
+        case kQsubParts + 1: generate_faces<tess::kQsub, true>(a); break;
+        case kTriParts: generate_faces<tess::kTri, false>(a); break;
+        default: generate_faces<tess::kTri, true>(a); break;
+    }
+}
+
+// The 32 coords from i0 on of a face of nc coords, located, written through shared memory (`stage`:
+// 160 words of the warp): whole sectors of the 20-byte records.
+__device__ __forceinline__ void locate_coords(const GenArgs &a, int N, int ptex0, float2 uv, int i0,
+                                              int nc, int64_t c0, int *stage, int lane) {
+    if (i0 + lane < nc) locate_coord(a, N, ptex0, uv.x, uv.y, stage + 5 * lane);
+    __syncwarp();
+    const int words = 5 * min(32, nc - i0);
+    int *out = a.patchCoords + 5 * (c0 + i0);
+#pragma unroll
+    for (int m = 0; m < 5; ++m)
+        if (lane + 32 * m < words) out[lane + 32 * m] = stage[lane + 32 * m];
+    __syncwarp();
+}
+
+// A face's nf facets at `from` (facets `step` words apart) moved by `delta` into its slice at
+// facet f0 of the output: word by word where both are packed, so that neighbouring lanes write
+// neighbouring words.
+template <int FS>
+__device__ __forceinline__ void move_facets(const GenArgs &a, const int *from, int step, int64_t f0,
+                                            int nf, int delta, int lane) {
+    int *to = a.facets + f0 * a.facetStride;
+    if (a.facetStride == FS && step == FS) {
+        for (int q = lane; q < nf * FS; q += 32) {
+            const int v = from[q];
+            to[q] = v >= 0 ? v + delta : v;
+        }
+        return;
+    }
+    for (int q = lane; q < nf; q += 32) {
+        const int *src = from + (int64_t)q * step;
+        int *d = to + (int64_t)q * a.facetStride;
+#pragma unroll
+        for (int c = 0; c < FS; ++c) {
+            const int v = src[c];
+            d[c] = v >= 0 ? v + delta : v;
+        }
+    }
+}
+
+// One warp per face: copies a shared pattern, or the slice of the face that owns its pattern,
+// into its own (coords as float2 pairs), and locates every coord of the face on the patch table.
 template <int FS>
 __global__ void __launch_bounds__(256) k_tess_finish(const GenArgs a) {
+    __shared__ int stages[8][160];
     const int lane = threadIdx.x & 31;
+    int *stage = stages[threadIdx.x >> 5];
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int f = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; f < a.numFaces; f += warps) {
         const int64_t c0 = a.co[f];
@@ -269,82 +348,42 @@ __global__ void __launch_bounds__(256) k_tess_finish(const GenArgs a) {
         const int N = a.faceSizes[f];
         const bool sh = uses_shared(a, N);
         const int own = sh ? f : owner_of(a, f);
-        if (!sh && own == f && !a.locate) continue;
+        const bool copy = sh || own != f;
+        if (!copy && !a.locate) continue;
         const int k = N - kFirstShared;
         const int ptex0 = a.locate ? (int)a.po[f] : 0;
-        if (!sh && own != f) {
-            // a copy of the owner's slice: same coords, facet indices moved by the difference
-            // of the two faces' first coords
-            const int64_t s0 = a.co[own];
-            for (int i = lane; i < nc; i += 32) {
-                const float *c = a.coords + (s0 + i) * a.coordStride;
-                float *d = a.coords + (c0 + i) * a.coordStride;
-                float u, v;
-                if (a.coordPairs) {
-                    const float2 uv = *reinterpret_cast<const float2 *>(c);
-                    *reinterpret_cast<float2 *>(d) = uv;
-                    u = uv.x;
-                    v = uv.y;
-                } else {
-                    u = c[0];
-                    v = c[1];
-                    d[0] = u;
-                    d[1] = v;
-                }
-                if (a.locate) locate_coord(a, N, ptex0, u, v, a.patchCoords + 5 * (c0 + i));
-            }
-            const int64_t f0 = a.fo[f], g0 = a.fo[own];
-            const int nf = (int)(a.fo[f + 1] - f0);
-            const int delta = a.offsetIndices ? (int)(c0 - s0) : 0;
-            for (int q = lane; q < nf; q += 32) {
-                const int *src = a.facets + (g0 + q) * a.facetStride;
-                int *d = a.facets + (f0 + q) * a.facetStride;
-#pragma unroll
-                for (int c = 0; c < FS; ++c) {
-                    const int v = src[c];
-                    d[c] = v >= 0 ? v + delta : v;
+        const int64_t s0 = sh ? 0 : a.co[own];
+        const float *from =
+            sh ? a.patCoords + 2 * (int64_t)a.patC[k] : a.coords + s0 * a.coordStride;
+        const int step = sh ? 2 : a.coordStride;
+        for (int i0 = 0; i0 < nc; i0 += 32) {
+            const int i = i0 + lane;
+            float2 uv = make_float2(0.0f, 0.0f);
+            if (i < nc) {
+                const float *c = from + (int64_t)i * step;
+                if (sh || a.coordPairs) uv = *reinterpret_cast<const float2 *>(c);
+                else uv = make_float2(c[0], c[1]);
+                if (copy) {
+                    float *d = a.coords + (c0 + i) * a.coordStride;
+                    if (a.coordPairs) {
+                        *reinterpret_cast<float2 *>(d) = uv;
+                    } else {
+                        d[0] = uv.x;
+                        d[1] = uv.y;
+                    }
                 }
             }
-        } else if (sh) {
-            const float2 *pc = reinterpret_cast<const float2 *>(a.patCoords) + a.patC[k];
-            for (int i = lane; i < nc; i += 32) {
-                const float2 uv = pc[i];
-                float *d = a.coords + (c0 + i) * a.coordStride;
-                if (a.coordPairs) {
-                    *reinterpret_cast<float2 *>(d) = uv;
-                } else {
-                    d[0] = uv.x;
-                    d[1] = uv.y;
-                }
-                if (a.locate) locate_coord(a, N, ptex0, uv.x, uv.y, a.patchCoords + 5 * (c0 + i));
-            }
-            const int64_t f0 = a.fo[f];
-            const int nf = (int)(a.fo[f + 1] - f0);
-            const int off = a.offsetIndices ? (int)c0 : 0;
-            const int *pf = a.patFacets + FS * a.patF[k];
-            for (int q = lane; q < nf; q += 32) {
-                int *d = a.facets + (f0 + q) * a.facetStride;
-#pragma unroll
-                for (int c = 0; c < FS; ++c) {
-                    const int v = pf[FS * q + c];
-                    d[c] = v >= 0 ? v + off : v;
-                }
-            }
-        } else {
-            for (int i = lane; i < nc; i += 32) {
-                const float *c = a.coords + (c0 + i) * a.coordStride;
-                float u, v;
-                if (a.coordPairs) {
-                    const float2 uv = *reinterpret_cast<const float2 *>(c);
-                    u = uv.x;
-                    v = uv.y;
-                } else {
-                    u = c[0];
-                    v = c[1];
-                }
-                locate_coord(a, N, ptex0, u, v, a.patchCoords + 5 * (c0 + i));
-            }
+            if (a.locate) locate_coords(a, N, ptex0, uv, i0, nc, c0, stage, lane);
         }
+        if (!copy) continue;
+        const int64_t f0 = a.fo[f];
+        const int nf = (int)(a.fo[f + 1] - f0);
+        if (sh)
+            move_facets<FS>(a, a.patFacets + FS * a.patF[k], FS, f0, nf,
+                            a.offsetIndices ? (int)c0 : 0, lane);
+        else
+            move_facets<FS>(a, a.facets + a.fo[own] * a.facetStride, a.facetStride, f0, nf,
+                            a.offsetIndices ? (int)(c0 - s0) : 0, lane);
     }
 }
 
@@ -864,10 +903,18 @@ extern "C" int GB300TessellationCount(int regularFaceSize, int numFaces, const i
         return fail(GB300_ERR_INVALID_ARGUMENT, "%s: null offsets or totals", who);
     cudaStream_t s = as_stream(stream);
     const int n1 = numFaces + 1;
-    int64_t *counts = nullptr;
-    if ((st = scratch_alloc((void **)&counts, sizeof(int64_t) * 3 * (size_t)n1, s, who)) !=
-        GB300_OK)
-        return st;
+    // one scan of the three counts together and one copy of the totals
+    const size_t nb = sizeof(Totals) * (size_t)n1;
+    size_t bytes = 0;
+    st = check_cuda(cub::DeviceScan::ExclusiveScan(nullptr, bytes, (Totals *)nullptr,
+                                                   (Totals *)nullptr, TotalsSum{},
+                                                   Totals{0, 0, 0}, n1, s),
+                    who);
+    if (st != GB300_OK) return st;
+    char *scratch = nullptr;
+    const size_t at = (2 * nb + 255) & ~size_t(255);
+    if ((st = scratch_alloc((void **)&scratch, at + bytes, s, who)) != GB300_OK) return st;
+    Totals *scan = (Totals *)(scratch + nb);
     CountArgs a;
     a.reg = regularFaceSize;
     a.numFaces = numFaces;
@@ -877,30 +924,25 @@ extern "C" int GB300TessellationCount(int regularFaceSize, int numFaces, const i
     a.faceSizes = faceSizes;
     a.rateOffsets = rateOffsets;
     a.rates = rates;
-    a.cc = counts;
-    a.fc = counts + n1;
-    a.pc = counts + 2 * (size_t)n1;
+    a.counts = (Totals *)scratch;
     k_tess_count<<<grid_for(n1, 256, 16), 256, 0, s>>>(a);
     count_launch();
     st = check_launch(who);
-    size_t bytes = 0;
-    void *tmp = nullptr;
     if (st == GB300_OK)
-        st = check_cuda(cub::DeviceScan::ExclusiveSum(nullptr, bytes, a.cc, coordOffsets, n1, s),
-                        who);
-    if (st == GB300_OK) st = scratch_alloc(&tmp, bytes, s, who);
-    int64_t *outs[3] = {coordOffsets, facetOffsets, ptexOffsets};
-    for (int k = 0; k < 3 && st == GB300_OK; ++k)
-        st = check_cuda(cub::DeviceScan::ExclusiveSum(tmp, bytes, counts + k * (size_t)n1,
-                                                      outs[k], n1, s),
+        st = check_cuda(cub::DeviceScan::ExclusiveScan(scratch + at, bytes, a.counts, scan,
+                                                       TotalsSum{}, Totals{0, 0, 0}, n1, s),
                         who);
     int64_t host[3] = {0, 0, 0};
-    for (int k = 0; k < 3 && st == GB300_OK; ++k)
-        st = check_cuda(cudaMemcpyAsync(host + k, outs[k] + numFaces, sizeof(int64_t),
-                                        cudaMemcpyDeviceToHost, s),
-                        who);
-    if (tmp) scratch_free(tmp, s);
-    scratch_free(counts, s);
+    if (st == GB300_OK) {
+        k_tess_offsets<<<grid_for(n1, 256, 16), 256, 0, s>>>(scan, n1, coordOffsets, facetOffsets,
+                                                            ptexOffsets);
+        count_launch();
+        if ((st = check_launch(who)) == GB300_OK)
+            st = check_cuda(cudaMemcpyAsync(host, scan + numFaces, sizeof(host),
+                                            cudaMemcpyDeviceToHost, s),
+                            who);
+    }
+    scratch_free(scratch, s);
     if (st == GB300_OK) st = check_cuda(cudaStreamSynchronize(s), who);
     if (st != GB300_OK) return st;
     for (int k = 0; k < 3; ++k) totals[k] = host[k];
@@ -1032,17 +1074,10 @@ extern "C" int GB300TessellationGenerate(
         // with shared patterns only polygons above 10 sides are generated per face: none for
         // a triangle scheme, only quad sub-face polygons for a quad scheme
         const int grid = grid_for(numFaces, 128, 16);
-        if (regularFaceSize == 3) {
-            if (!a.shared) {
-                k_tess_generate<tess::kTri><<<grid, 128, 0, s>>>(a);
-                count_launch();
-            }
-        } else {
-            if (!a.shared) {
-                k_tess_generate<tess::kQuad><<<grid, 128, 0, s>>>(a);
-                count_launch();
-            }
-            k_tess_generate<tess::kQsub><<<grid, 128, 0, s>>>(a);
+        if (regularFaceSize == 4 || !a.shared) {
+            const int first = regularFaceSize == 3 ? kTriParts : a.shared ? kQsubParts : kQuadParts;
+            const int parts = regularFaceSize == 4 && !a.shared ? 4 : 2;
+            k_tess_generate<<<dim3(grid, parts), 128, 0, s>>>(a, first);
             count_launch();
         }
         st = check_launch(who);
