@@ -200,5 +200,31 @@ __device__ __forceinline__ void eval_one12(const A &a, int i, int n, const int *
     }
 }
 
+// The rows of a warp's 32 stencils (destination rows in `rows`, -1: none), `length` floats at `dst`
+// that no vector store can take, collected in `scratch` (32 * length floats of shared memory) and
+// written so that neighbouring lanes write neighbouring elements: one store per 32 elements.  By
+// their lanes every element is a store of its own to each row's sector (rows of 9-11 floats in the
+// batched scene: 65.6 M sectors written for 8.4 M).  magic: 65536 / length + 1.
+template <int CW>
+__device__ __forceinline__ void store_rows(float *dst, int stride, int length, unsigned magic,
+                                           const int *rows, float *scratch, int lane,
+                                           const float (&acc)[CW]) {
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < CW; ++c)
+        if (c < length) scratch[lane * length + c] = acc[c];
+    __syncwarp();
+    for (int e = lane; e < 32 * length; e += 32) {
+        const int r = (int)((unsigned)e * magic >> 16);
+        const int row = rows[r];
+        if (row >= 0) st_stream(dst + (size_t)row * stride + (e - r * length), scratch[e]);
+    }
+}
+
+// Orders this thread's shared-memory accesses before later bulk copies into the same memory.
+__device__ __forceinline__ void fence_async() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 }  // namespace tma
 }  // namespace gb300

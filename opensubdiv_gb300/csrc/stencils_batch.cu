@@ -174,7 +174,7 @@ constexpr int kUnits = 3;  // every job reads its table's unit layout (mode 3)
 // index and weight from the stage (slot base `slot0`) or, for a slice wider than the stage,
 // from global memory; columns per pass by job class.
 template <int CLS>
-__device__ __forceinline__ void slice_warp(const Job &j, const Meta &m, int wl, const int *sidx,
+__device__ __forceinline__ void slice_warp(const Job &j, const Meta &m, int wl, int *sidx,
                                            const float *sw, const int *ssz, const int *srow,
                                            int lane, uint64_t pol_src, uint64_t pol_stream) {
     constexpr bool WIDE = CLS == kWide;
@@ -237,6 +237,11 @@ __device__ __forceinline__ void slice_warp(const Job &j, const Meta &m, int wl, 
                 if (j0 + q < n)
 #pragma unroll
                     for (int c = 0; c < CW; ++c) acc[c] = fmaf(wk[q], x[q][c], acc[c]);
+        }
+        if (m.staged && !j.vecDst[0] && j.length <= CW && width >= j.length) {
+            tma::store_rows(j.dst[0], j.dstStride[0], j.length, 65536u / (unsigned)j.length + 1,
+                            srow + wl * 32, reinterpret_cast<float *>(sidx + base - lane), lane, acc);
+            continue;
         }
         if (row < 0) continue;
         float *d = j.dst[0] + (size_t)row * j.dstStride[0] + c0;
@@ -451,6 +456,7 @@ __global__ void __launch_bounds__(kThreads, (Ring<CLS, SLICED>::kMinBlocks))
                     stencil_warp(j, i, n, o, nullptr, nullptr, lane, pol_src);
             }
         }
+        if constexpr (SLICED) tma::fence_async();
         __syncwarp();
         if (lane == 0) bar_arrive(&empty[stage]);
     }

@@ -292,7 +292,7 @@ struct SellCfg {
     static constexpr int kSlots = kTwo ? 4096 : NW <= 3 ? 2048 : 1024;  // slots per stage
     static constexpr int kSpt = kSlots / 512;  // slices per tile (staged up to width 16)
     static constexpr size_t kStageBytes = (size_t)kSpt * 32 * 8 + (size_t)kSlots * 4 * (1 + NW);
-    static constexpr int kRing = kTwo ? 2 : NW >= 4 ? 4 : kStages;
+    static constexpr int kRing = kTwo ? 2 : NW >= 4 && !(NW == 6 && VW == kNarrow) ? 4 : kStages;
     static constexpr size_t kSmem = kRing * kStageBytes + 256;
 };
 
@@ -306,6 +306,7 @@ struct SellArgs {
     int dstStride[6];
     int outOf[6];
     int vecDst[6];
+    unsigned magic;  // 65536 / length + 1
 };
 
 struct SellMeta {
@@ -374,15 +375,16 @@ __device__ __forceinline__ void store_cols(const SellArgs &a, int o, int row, in
 // the refine pass, 12-wide rows 0.372 -> 0.356 ms), and for 3 outputs over rows of up to 4
 // floats; two otherwise (more would spill), one for 6 outputs.
 template <int NW, int VW>
-__global__ void __launch_bounds__(kThreads, NW >= 6 ? 1 : (NW == 1 || VW == kNarrow) ? 3 : 2)
+__global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow) ? 3 : NW >= 6 && VW != kNarrow ? 1 : 2)
     k_stencils_sell(const SellArgs a) {
     extern __shared__ __align__(128) char smem[];
     using C = SellCfg<NW, VW>;
     constexpr int S = C::kRing, SPT = C::kSpt;
-    constexpr int G = 8 / SPT;          // consumer groups (one warp per slice of a tile)
-    constexpr int GT = kConsumers / G;  // threads per group
-    constexpr int GW = GT / 32;         // warps per group (= SPT)
-    static_assert(G >= 1 && G <= S && GW == SPT, "consumer groups");
+    // consumer groups (one warp per slice of a tile), no more than the ring has stages: a group
+    // waits for its stage's use `it / S` by parity, which tells it from the use before only
+    constexpr int G = 8 / SPT < S ? 8 / SPT : S;
+    constexpr int GW = SPT;  // warps per group
+    static_assert(G >= 1 && G <= S && G * GW <= kConsumers / 32, "consumer groups");
     __shared__ __align__(8) uint64_t full[S], empty[S];
     __shared__ SellMeta meta[S];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -439,6 +441,7 @@ __global__ void __launch_bounds__(kThreads, NW >= 6 ? 1 : (NW == 1 || VW == kNar
     // consumers: group g takes this CTA's tiles it = g, g + G, ...; warp wg of the group takes
     // slice wg of the tile
     const int grp = warp / GW, wg = warp - grp * GW;
+    if (grp >= G) return;
     // entry steps gathered together, columns per pass
     constexpr int R = VW == kNarrow ? (NW == 1 ? 6 : 4) : VW == 12 ? 2 : NW <= 3 ? 4 : 2;
     constexpr int CW = VW == 12 ? 12 : VW == kNarrow ? 4 : 8;
@@ -464,31 +467,36 @@ __global__ void __launch_bounds__(kThreads, NW >= 6 ? 1 : (NW == 1 || VW == kNar
                 for (int k = 0; k < NW; ++k)
 #pragma unroll
                     for (int c = 0; c < CW; ++c) acc[k][c] = 0.0f;
+                // Steps past a lane's last entry: with one output they are skipped; with more they
+                // load that entry again and add nothing, because the registers of a load that is
+                // predicated off stay live around the loop (3 outputs of 8-wide rows 75.8 -> 73.8
+                // us; one output of Loop stencils, whose sizes differ more, 24.2 -> 24.6 us).
+                constexpr bool SKIP = NW == 1;
+                const int last = max(n - 1, 0);
                 for (int j0 = 0; j0 < width; j0 += R) {
                     int ids[R];
                     float wk[R][NW];
 #pragma unroll
                     for (int q = 0; q < R; ++q) {
-                        const int j = j0 + q;
-                        if (j < n) {
-                            if (m.staged) {
-                                ids[q] = sidx[base + j * 32];
+                        const int j = SKIP ? j0 + q : min(j0 + q, last);
+                        if (SKIP && j >= n) continue;
+                        if (m.staged) {
+                            ids[q] = sidx[base + j * 32];
 #pragma unroll
-                                for (int k = 0; k < NW; ++k)
-                                    wk[q][k] = sw[(size_t)k * C::kSlots + base + j * 32];
-                            } else {
-                                ids[q] = ld_stream(a.idx + b0 + lane + (size_t)j * 32, pol_stream);
+                            for (int k = 0; k < NW; ++k)
+                                wk[q][k] = sw[(size_t)k * C::kSlots + base + j * 32];
+                        } else {
+                            ids[q] = ld_stream(a.idx + b0 + lane + (size_t)j * 32, pol_stream);
 #pragma unroll
-                                for (int k = 0; k < NW; ++k)
-                                    wk[q][k] = ld_stream(a.w[k] + b0 + lane + (size_t)j * 32,
-                                                         pol_stream);
-                            }
+                            for (int k = 0; k < NW; ++k)
+                                wk[q][k] = ld_stream(a.w[k] + b0 + lane + (size_t)j * 32,
+                                                     pol_stream);
                         }
                     }
                     float x[R][CW];
 #pragma unroll
                     for (int q = 0; q < R; ++q)
-                        if (j0 + q < n) gather_cols<VW>(a, ids[q], c0, pol_src, x[q]);
+                        if (!SKIP || j0 + q < n) gather_cols<VW>(a, ids[q], c0, pol_src, x[q]);
 #pragma unroll
                     for (int q = 0; q < R; ++q)
                         if (j0 + q < n)
@@ -498,12 +506,24 @@ __global__ void __launch_bounds__(kThreads, NW >= 6 ? 1 : (NW == 1 || VW == kNar
                                 for (int c = 0; c < CW; ++c)
                                     acc[k][c] = fmaf(wk[q][k], x[q][c], acc[k][c]);
                 }
-                if (row >= 0) {
+                // Narrow rows that no vector store takes leave through the slice's own part of the
+                // stage, which nothing reads any more after the last column pass, where several
+                // outputs make it worth it (six of xyz 38.9 -> 34.9 us); one output of 5-wide rows
+                // and three of 8-wide ones took 0.4 and 2.6 us longer for the extra code.
+                const bool collect =
+                    VW == kNarrow && NW > 1 && m.staged && a.length <= CW && width >= a.length;
 #pragma unroll
-                    for (int k = 0; k < NW; ++k) store_cols(a, a.outOf[k], row, c0, acc[k]);
+                for (int k = 0; k < NW; ++k) {
+                    const int o = a.outOf[k];
+                    if (collect && !a.vecDst[o])
+                        store_rows(a.dst[o], a.dstStride[o], a.length, a.magic, sor + wg * 32,
+                                   reinterpret_cast<float *>(sidx + base - lane), lane, acc[k]);
+                    else if (row >= 0)
+                        store_cols(a, o, row, c0, acc[k]);
                 }
             }
         }
+        if (VW == kNarrow && NW > 1) fence_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[st]);
     }
@@ -605,6 +625,7 @@ int eval_stencils_sell(const SellTable &t, const float *src, float *const *dst,
     a.src = src;
     a.srcStride = srcStride;
     a.length = length;
+    a.magic = 65536u / (unsigned)length + 1;
     a.sz = t.sz;
     a.sliceSlot = t.sliceSlot;
     a.idx = t.idx;
@@ -628,8 +649,15 @@ int eval_stencils_sell(const SellTable &t, const float *src, float *const *dst,
     int r;
     if ((nw == 1 || nw == 3) && vw >= 4 && length > 8 && length <= 12) {
         r = nw == 1 ? tma::launch_sell<1, 12>(a, s) : tma::launch_sell<3, 12>(a, s);
-    } else if ((nw == 1 || nw == 3) && vw >= 4 && length <= 4) {
-        r = nw == 1 ? tma::launch_sell<1, tma::kNarrow>(a, s) : tma::launch_sell<3, tma::kNarrow>(a, s);
+    } else if (vw >= 4 && length <= 4) {
+        switch (nw) {
+            case 1: r = tma::launch_sell<1, tma::kNarrow>(a, s); break;
+            case 2: r = tma::launch_sell<2, tma::kNarrow>(a, s); break;
+            case 3: r = tma::launch_sell<3, tma::kNarrow>(a, s); break;
+            case 4: r = tma::launch_sell<4, tma::kNarrow>(a, s); break;
+            case 5: r = tma::launch_sell<5, tma::kNarrow>(a, s); break;
+            default: r = tma::launch_sell<6, tma::kNarrow>(a, s); break;
+        }
     } else {
         switch (nw * 10 + vw) {
 #define GB300_SELL_CASES(NW)                                   \

@@ -279,8 +279,8 @@ __device__ __forceinline__ void generate_faces(const GenArgs &a) {
 
 // Blocks of row y of the grid generate part `first` + y.  A mesh has few distinct patterns, so the
 // launch lasts as long as one thread takes for its longest part: the parts -- two kinds of face,
-// coords and facets -- run at the same time, in one launch (41 + 23 us as a launch per kind of
-// both, and 28 us, for the per-edge rates of 69 k faces).  Each block's code is one part's.
+// coords and facets -- run at the same time, in one launch (a launch per kind, each thread coords and facets:
+// 41 + 23 us for the per-edge rates of 69 k faces; now 37 us).  Each block's code is one part's.
 constexpr int kQuadParts = 0, kQsubParts = 2, kTriParts = 4;
 
 __global__ void __launch_bounds__(128, 8) k_tess_generate(const GenArgs a, int first) {
