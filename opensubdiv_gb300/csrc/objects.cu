@@ -353,7 +353,9 @@ int table_eval(const GB300StencilTable *t, const float *src, float *const *dIn, 
                         "weights",
                         k);
     }
-    if (t->unit.numSlices > 0 && d[0] && src && units_take(src, srcStride, d[0], st[0]))
+    if (t->unit.numStencils >= kUnitCall && d[0] && src && units_take(src, srcStride) &&
+        (!units_collect(d[0], st[0]) ||
+         (t->unit.regular && t->unit.numStencils >= kUnitAnyRow)))
         return eval_stencils_units(t->unit, src, d[0], st[0], length, srcStride, s,
                                    "GB300StencilTableEval");
     if (t->sell.numSlices > 0 && t->sell.idx) {

@@ -168,7 +168,8 @@ __device__ __forceinline__ void tile_threads12(const Job &j, const Meta &m, cons
 // wide over 16-byte aligned rows (one 12-column pass), at most 4 floats over 16-byte aligned
 // rows (one 4-column pass; sliced batches only).
 constexpr int kAny = 0, kWide = 1, kNarrow = 2;
-constexpr int kUnits = 3;  // every job reads its table's unit layout (mode 3)
+// every job reads its table's unit layout (mode 3) and writes 16-byte aligned rows, or any rows
+constexpr int kUnits = 3, kUnitsCollect = 4;
 
 // One slice of a sliced job by one warp (lane = stencil): entry j of the 32 stencils at a time,
 // index and weight from the stage (slot base `slot0`) or, for a slice wider than the stage,
@@ -464,6 +465,7 @@ __global__ void __launch_bounds__(kThreads, (Ring<CLS, SLICED>::kMinBlocks))
 
 // Unit jobs: the slices of every job's unit layout (units.h), one list over all of them, as the
 // table kernel (stencils_units.cu) takes those of one table.
+template <bool COLLECT>
 __global__ void __launch_bounds__(units::kThreads, 1) k_stencils_batch_units(const Args a) {
     using namespace units;
     extern __shared__ __align__(128) char smem[];
@@ -499,7 +501,7 @@ __global__ void __launch_bounds__(units::kThreads, 1) k_stencils_batch_units(con
     };
     claim();
     Feed f;
-    Far far{reinterpret_cast<float4 *>(bytes + (size_t)kUnitRing * 128), q.far};
+    Far far = warp_far(bytes, q.far);
     for (;; ++f.popped) {
         while (more && f.room(q, d.w)) {
             if (lane == 0) slotJob[warp][f.pushed % kAhead] = jc;
@@ -517,7 +519,7 @@ __global__ void __launch_bounds__(units::kThreads, 1) k_stencils_batch_units(con
             int dstStride[1], srcStride, length;
         };
         const View v{j.src, {j.dst[0]}, {j.dstStride[0]}, j.srcStride, j.length};
-        if (!consume(v, q, bytes, reinterpret_cast<const char *>(j.slIdx), far, s, lane,
+        if (!consume<COLLECT>(v, q, bytes, reinterpret_cast<const char *>(j.slIdx), far, s, lane,
                      unit_shift(v.length), pol_stream, a.status))
             return;
         __syncwarp();
@@ -642,15 +644,17 @@ int plan_tiles(Job *jobs, const double *meanSize, int n, int tileStencils, int w
 int set_smem_attribute() {
     static std::atomic<uint64_t> attr{0};  // devices whose function attribute is set
     return once_per_device(attr, [] {
-        void (*const kernels[6])(Args) = {
+        void (*const kernels[7])(Args) = {
             k_stencils_batch<kAny, false>, k_stencils_batch<kWide, false>,
             k_stencils_batch<kAny, true>, k_stencils_batch<kWide, true>,
-            k_stencils_batch<kNarrow, true>, k_stencils_batch_units};
-        const size_t bytes[6] = {Ring<kAny, false>::kSmem, Ring<kWide, false>::kSmem,
+            k_stencils_batch<kNarrow, true>, k_stencils_batch_units<false>,
+            k_stencils_batch_units<true>};
+        const size_t bytes[7] = {Ring<kAny, false>::kSmem, Ring<kWide, false>::kSmem,
                                  Ring<kAny, true>::kSmem, Ring<kWide, true>::kSmem,
-                                 Ring<kNarrow, true>::kSmem, units::kSmemBytes};
+                                 Ring<kNarrow, true>::kSmem, units::kSmemBytes,
+                                 units::kSmemBytes};
         int st = GB300_OK;
-        for (int k = 0; k < 6 && st == GB300_OK; ++k)
+        for (int k = 0; k < 7 && st == GB300_OK; ++k)
             st = check_cuda(cudaFuncSetAttribute(kernels[k],
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)bytes[k]),
@@ -665,10 +669,10 @@ int launch_jobs(const Job *dJobs, const int *dTileBase, int n, int numTiles, int
     int st = set_smem_attribute();
     if (st != GB300_OK) return st;
     if (numTiles == 0) return ok();
-    if (cls == kUnits) {
+    if (cls == kUnits || cls == kUnitsCollect) {
         Args a{dJobs, dTileBase, n, numTiles, dCounter, dStatus, 0};
-        k_stencils_batch_units<<<std::min(numTiles, num_sms()), units::kThreads,
-                                 units::kSmemBytes, s>>>(a);
+        auto kern = cls == kUnits ? k_stencils_batch_units<false> : k_stencils_batch_units<true>;
+        kern<<<std::min(numTiles, num_sms()), units::kThreads, units::kSmemBytes, s>>>(a);
         count_launch();
         return check_launch("batched EvalStencils");
     }
@@ -736,13 +740,13 @@ uint64_t work_signature(const std::vector<Job> &jobs, const std::vector<double> 
 using namespace gb300;
 using namespace gb300::batch;
 
-constexpr int kParts = 4;
+constexpr int kParts = 5;
 
 struct GB300StencilBatch {
     // in launch order, one launch per part: the general jobs, the jobs at most 4 floats wide
     // over 16-byte aligned rows (sliced batches: the 4-column instantiation), the jobs 9-12
     // floats wide over 16-byte aligned rows (the 12-wide instantiation), and, of a sliced batch,
-    // the jobs that the unit layout takes; each part largest first
+    // the jobs that the unit layout takes, by their output rows; each part largest first
     std::vector<Job> jobs;
     std::vector<double> mean;  // mean stencil size per job (same order)
     int part[kParts] = {};     // jobs per part
@@ -785,8 +789,8 @@ namespace {
 std::mutex g_tuneLock;
 std::map<uint64_t, Config> g_tuned;  // work signature -> best config
 
-constexpr int kPartClass[kParts] = {kAny, kNarrow, kWide, kUnits};
-constexpr int kPartCounter[kParts] = {0, 3, 2, 0};  // the last one claims within its CTAs
+constexpr int kPartClass[kParts] = {kAny, kNarrow, kWide, kUnits, kUnitsCollect};
+constexpr int kPartCounter[kParts] = {0, 3, 2, 0, 0};  // the last two claim within their CTAs
 
 // Applies b->cfg: job modes, tile sizes and the tile prefixes, uploaded to the device.
 int upload_plan(GB300StencilBatch *b, cudaStream_t s) {
@@ -962,7 +966,7 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
     for (size_t k = 0; k < b->jobs.size(); ++k) {
         Job &j = b->jobs[k];
         if (!b->sliced || units[k]->numSlices == 0 ||
-            !units_take(j.src, j.srcStride, j.dst[0], j.dstStride[0]))
+            !units_take(j.src, j.srcStride))
             continue;
         j.mode = 3;
         j.slSz = reinterpret_cast<const int *>(units[k]->slice);
@@ -976,7 +980,7 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
     {
         const bool sliced = b->sliced;
         auto part_of = [sliced](const Job &j) {
-            if (j.mode == 3) return 3;
+            if (j.mode == 3) return units_collect(j.dst[0], j.dstStride[0]) ? 4 : 3;
             if (j.vw >= 4 && j.length > 8 && j.length <= 12) return 2;
             if (sliced && j.vw >= 4 && j.length <= 4) return 1;
             return 0;

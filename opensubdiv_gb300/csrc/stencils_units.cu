@@ -19,6 +19,7 @@ struct Args {
     int dstStride[1];
 };
 
+template <bool COLLECT>
 __global__ void __launch_bounds__(kThreads, 1) k_stencils_units(const Args a) {
     extern __shared__ __align__(128) char smem[];
     __shared__ Queue queue[kWarps];
@@ -45,7 +46,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_stencils_units(const Args a) {
     };
     claim();
     Feed f;
-    Far far{reinterpret_cast<float4 *>(bytes + (size_t)kUnitRing * 128), q.far};
+    Far far = warp_far(bytes, q.far);
     for (;; ++f.popped) {
         while (more && f.room(q, d.w)) {
             f.push(q, bytes, a.blob, d, lane, pol_stream);
@@ -54,7 +55,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_stencils_units(const Args a) {
         if (f.popped == f.pushed) return;
         const int s = f.popped % kAhead;
         if (!ring::wait(&q.full[s], (uint32_t)(f.popped / kAhead) & 1, a.status)) return;
-        if (!consume(a, q, bytes, a.blob, far, s, lane, a.shift, pol_stream, a.status))
+        if (!consume<COLLECT>(a, q, bytes, a.blob, far, s, lane, a.shift, pol_stream, a.status))
             return;
         __syncwarp();
     }
@@ -62,8 +63,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_stencils_units(const Args a) {
 
 }  // namespace units
 
-bool units_take(const float *src, int srcStride, const float *dst, int dstStride) {
-    return (((uintptr_t)src | (uintptr_t)dst) & 15) == 0 && (srcStride | dstStride) % 4 == 0;
+bool units_take(const float *src, int srcStride) {
+    return ((uintptr_t)src & 15) == 0 && srcStride % 4 == 0;
+}
+
+bool units_collect(const float *dst, int dstStride) {
+    return ((uintptr_t)dst & 15) != 0 || dstStride % 4 != 0;
 }
 
 int eval_stencils_units(const UnitTable &t, const float *src, float *dst, int dstStride,
@@ -73,14 +78,22 @@ int eval_stencils_units(const UnitTable &t, const float *src, float *dst, int ds
         return fail(GB300_ERR_INVALID_ARGUMENT, "%s: bad source", who);
     if (dstStride < length)
         return fail(GB300_ERR_INVALID_ARGUMENT, "%s: output 0 stride / weights", who);
-    if (!units_take(src, srcStride, dst, dstStride))
+    if (!units_take(src, srcStride))
         return fail(GB300_ERR_INVALID_ARGUMENT, "%s: rows are not 16-byte aligned", who);
+    auto kern = units_collect(dst, dstStride) ? units::k_stencils_units<true>
+                                              : units::k_stencils_units<false>;
     static std::atomic<uint64_t> attr{0};
     int r = once_per_device(attr, [&] {
-        return check_cuda(cudaFuncSetAttribute(units::k_stencils_units,
+        const int st = check_cuda(cudaFuncSetAttribute(units::k_stencils_units<true>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       units::kSmemBytes),
+                                  who);
+        return st != GB300_OK ? st
+                              : check_cuda(cudaFuncSetAttribute(
+                                               units::k_stencils_units<false>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                units::kSmemBytes),
-                          who);
+                                           who);
     });
     units::Args a{};
     if (r != GB300_OK || (r = status_word_address(&a.status)) != GB300_OK) return r;
@@ -93,7 +106,7 @@ int eval_stencils_units(const UnitTable &t, const float *src, float *dst, int ds
     a.numSlices = t.numSlices;
     a.dst[0] = dst;
     a.dstStride[0] = dstStride;
-    units::k_stencils_units<<<min(a.numSlices, num_sms()), units::kThreads, units::kSmemBytes, s>>>(a);
+    kern<<<min(a.numSlices, num_sms()), units::kThreads, units::kSmemBytes, s>>>(a);
     count_launch();
     return check_launch(who);
 }

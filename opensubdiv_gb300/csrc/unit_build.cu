@@ -202,6 +202,7 @@ struct Slices {
     const int *order;
     const long long *start;   // blob offset / 128 (fill)
     long long *bytes;         // blob size / 128 (size)
+    unsigned long long *shared;  // stencils of uniform slices
     int4 *slice;
     char *blob;
 };
@@ -246,6 +247,7 @@ __global__ void __launch_bounds__(256) k_unit_sizes(const Slices a, int4 *meta) 
             const long long w = (long long)m * padded(n), head = m + (long long)n;
             meta[s] = make_int4(0, n, m | (same ? 256 : 0), 0);
             a.bytes[s] = same ? head + (w + 31) / 32 : head + 1 + w;
+            if (same) atomicAdd(a.shared, 32ull * m);
         }
     }
 }
@@ -427,14 +429,21 @@ int build_units(int n, const int *sizes, const int *offsets, const int *indices,
     count_launch();
     sort(skey, skey2, siota, at, ns, 32);
     if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
-    Slices a{c, ns, at, firstOf, seg2, unit, pos, count, order, start, bytes, nullptr, nullptr};
-    if (check_cuda(cudaMemsetAsync(bytes + ns, 0, 8, s), who) != GB300_OK) return GB300_ERR_CUDA;
+    u64 *shared = tmp.get<u64>(1);
+    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    Slices a{c,     ns,    at,      firstOf, seg2,    unit, pos, count,
+             order, start, bytes, shared,  nullptr, nullptr};
+    if (check_cuda(cudaMemsetAsync(bytes + ns, 0, 8, s), who) != GB300_OK ||
+        check_cuda(cudaMemsetAsync(shared, 0, 8, s), who) != GB300_OK)
+        return GB300_ERR_CUDA;
     k_unit_sizes<<<grid_of((long long)ns * 32, 256), 256, 0, s>>>(a, meta);
     count_launch();
     scan(bytes, start, ns + 1);
     if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
     long long total = 0;
-    if ((st = check_launch(who)) != GB300_OK || (st = read(&total, start + ns)) != GB300_OK)
+    u64 sharing = 0;
+    if ((st = check_launch(who)) != GB300_OK || (st = read(&total, start + ns)) != GB300_OK ||
+        (st = read(&sharing, shared)) != GB300_OK)
         return st;
     if (total > INT_MAX) return GB300_ERR_UNSUPPORTED;
     auto fail_all = [&](int code) {
@@ -454,6 +463,8 @@ int build_units(int n, const int *sizes, const int *offsets, const int *indices,
     if (check_launch(who) != GB300_OK || check_cuda(cudaStreamSynchronize(s), who) != GB300_OK)
         return fail_all(GB300_ERR_CUDA);
     t.numSlices = ns;
+    t.regular = sharing >= (u64)n / 2;
+    t.numStencils = n;
     t.slice = a.slice;
     t.blob = a.blob;
     return ok();

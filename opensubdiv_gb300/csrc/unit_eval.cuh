@@ -1,6 +1,7 @@
 // Evaluation of one slice of the unit layout (units.h) by one warp, shared by the table kernel
 // (stencils_units.cu) and the batched kernel (stencils_batch.cu).  `A` is the launch's argument
-// view: src, srcStride, length, dst[0], dstStride[0]; the rows of both are 16-byte aligned.
+// view: src (rows 16-byte aligned), srcStride, length, dst[0], dstStride[0].  COLLECT: the rows of
+// dst are not 16-byte aligned.
 //
 // A lane holds 4 columns of the up to 16 source rows of its unit's list in registers and runs
 // through the unit's stencils: the rows are gathered once for all of them, 16 loads in flight at
@@ -40,6 +41,33 @@ __device__ __forceinline__ void store_quad(const A &a, int row, int c0, const fl
     if (rem > 2) st_stream(d + 2, v.z);
 }
 
+constexpr int kOut = 128;  // floats of one stencil of all units evaluated at a time
+
+// Rows of any other layout (xyz above all): the columns [c, c + width) of one stencil of `units` units,
+// collected in `out` and written so that neighbouring lanes write neighbouring elements.  The lanes'
+// own stores would take one for every element, each to another row's sector.  magic: 65536 / width + 1.
+template <class A>
+__device__ __forceinline__ void store_collected(const A &a, float *out, const int *rows, int units,
+                                                int shift, int c, int width, unsigned magic,
+                                                int lane, const float4 &v) {
+    const int at = 4 * (lane & ((1 << shift) - 1));
+    float *d = out + (lane >> shift) * width + at;
+    if (at < width) d[0] = v.x;
+    if (at + 1 < width) d[1] = v.y;
+    if (at + 2 < width) d[2] = v.z;
+    if (at + 3 < width) d[3] = v.w;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < kOut / 32; ++i) {
+        const int e = lane + 32 * i, u = (int)((unsigned)e * magic >> 16);
+        if (e >= units * width) break;
+        const int row = rows[u];
+        if (row >= 0)
+            st_stream(a.dst[0] + (size_t)row * a.dstStride[0] + c + (e - u * width), out[e]);
+    }
+    __syncwarp();
+}
+
 __device__ __forceinline__ float4 load_far(const float4 *p) {  // weights, read once
     float4 v;
     asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -55,6 +83,7 @@ constexpr int kFarBlock = 128;
 
 struct Far {
     float4 *buf;
+    float *out;  // kOut floats, where output rows are collected
     uint64_t *full;
     int issued = 0, used = 0;  // blocks, over all slices
 };
@@ -82,7 +111,7 @@ __device__ __forceinline__ void gather(const A &a, const int *idx, int j0, int k
 // `far`, a block of 2^shift stencils at a time, as many blocks ahead as there are.  NQ =
 // ceil(n / 4).  One loop serves both kinds: with one body per kind the instruction cache did not
 // hold the bodies that the warps of an SM run at the same time.
-template <int NQ, class A>
+template <int NQ, bool COLLECT, class A>
 __device__ __forceinline__ bool slice(const A &a, const char *p, const float4 *weights, Far &far,
                                       int n, int m, bool uni, int lane, int shift,
                                       uint64_t pol_stream, int *status) {
@@ -125,6 +154,8 @@ __device__ __forceinline__ bool slice(const A &a, const char *p, const float4 *w
         for (int c = 0; c < a.length; c += 4 << shift) {
             const int c0 = c + 4 * (lane & ((1 << shift) - 1));
             const bool on = c0 < a.length;
+            const int width = min(4 << shift, a.length - c);
+            const unsigned magic = COLLECT ? 65536u / (unsigned)width + 1 : 0;
             float4 x[4 * NQ];
             gather<NQ>(a, idx + u, 0, on ? k : 0, c0, x);
 #pragma unroll 1
@@ -140,7 +171,7 @@ __device__ __forceinline__ bool slice(const A &a, const char *p, const float4 *w
                 const int end = min(s + per, m);
 #pragma unroll 1
                 for (; s < end; ++s) {
-                    const int row = rows[32 * s + u];
+                    const int row = COLLECT ? 0 : rows[32 * s + u];
                     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
                     for (int q = 0; q < NQ; ++q, w += qstep) {
@@ -150,7 +181,11 @@ __device__ __forceinline__ bool slice(const A &a, const char *p, const float4 *w
                         add_row(v.z, x[4 * q + 2], acc);
                         add_row(v.w, x[4 * q + 3], acc);
                     }
-                    if (on && row >= 0) store_quad(a, row, c0, acc);
+                    if constexpr (COLLECT)
+                        store_collected(a, far.out, rows + 32 * s + u0, units, shift, c, width,
+                                        magic, lane, acc);
+                    else if (on && row >= 0)
+                        store_quad(a, row, c0, acc);
                 }
                 if (!uni) {
                     __syncwarp();
@@ -164,9 +199,9 @@ __device__ __forceinline__ bool slice(const A &a, const char *p, const float4 *w
 }
 
 // A slice of single stencils of more than 16 entries, 16 at a time; p may be in global memory.
-template <class A>
+template <bool COLLECT, class A>
 __device__ __forceinline__ void long_slice(const A &a, const int *rows, const float4 *far, int n,
-                                           int lane, int shift) {
+                                           float *out, int lane, int shift) {
     const int nq = (n + 3) / 4;
 #pragma unroll 1
     for (int u = lane >> shift; u < 32; u += 32 >> shift) {
@@ -195,7 +230,13 @@ __device__ __forceinline__ void long_slice(const A &a, const int *rows, const fl
                     add_row(v[q].w, x[4 * q + 3], acc);
                 }
             }
-            if (on) store_quad(a, row, c0, acc);
+            if constexpr (COLLECT) {
+                const int width = min(4 << shift, a.length - c);
+                store_collected(a, out, rows + u - (lane >> shift), 32 >> shift, shift, c, width,
+                                65536u / (unsigned)width + 1, lane, acc);
+            } else if (on) {
+                store_quad(a, row, c0, acc);
+            }
         }
     }
 }

@@ -17,8 +17,14 @@ namespace units {
 constexpr int kWarps = 16;  // one CTA per SM: 128 registers a thread
 constexpr int kThreads = kWarps * 32;
 constexpr int kAhead = 2;  // slices a warp has in its ring
-constexpr int kWarpBytes = kUnitRing * 128 + kFarBlocks * kFarBlock * 16;  // ring, weights
+constexpr int kWarpBytes = kUnitRing * 128 + kFarBlocks * kFarBlock * 16 + kOut * 4;
 constexpr int kSmemBytes = kWarps * kWarpBytes;
+
+// A warp's part of the shared memory: its ring, its weights in flight, its output rows.
+__device__ __forceinline__ Far warp_far(char *bytes, uint64_t *full) {
+    return Far{reinterpret_cast<float4 *>(bytes + (size_t)kUnitRing * 128),
+               reinterpret_cast<float *>(bytes + kWarpBytes - kOut * 4), full};
+}
 
 struct Queue {
     uint64_t full[kAhead];
@@ -90,7 +96,7 @@ struct Feed {
 
 // The slice in slot s, once full.  shift: log2 of the lanes that share a unit.  False when a wait
 // for its weights expired.
-template <class A>
+template <bool COLLECT, class A>
 __device__ __forceinline__ bool consume(const A &a, const Queue &q, const char *bytes,
                                         const char *blob, Far &far, int s, int lane, int shift,
                                         uint64_t pol_stream, int *status) {
@@ -101,19 +107,19 @@ __device__ __forceinline__ bool consume(const A &a, const Queue &q, const char *
     const bool uni = (d.z & 256) != 0;
     switch (d.y > kUnitList ? 5 : (d.y + 3) >> 2) {
         case 4:
-            return slice<4>(a, p, w, far, d.y, m, uni, lane, shift, pol_stream, status);
+            return slice<4, COLLECT>(a, p, w, far, d.y, m, uni, lane, shift, pol_stream, status);
         case 3:
-            return slice<3>(a, p, w, far, d.y, m, uni, lane, shift, pol_stream, status);
+            return slice<3, COLLECT>(a, p, w, far, d.y, m, uni, lane, shift, pol_stream, status);
         case 2:
-            return slice<2>(a, p, w, far, d.y, m, uni, lane, shift, pol_stream, status);
+            return slice<2, COLLECT>(a, p, w, far, d.y, m, uni, lane, shift, pol_stream, status);
         case 5:
-            long_slice(a,
+            long_slice<COLLECT>(a,
                             reinterpret_cast<const int *>(
                                 d.z & kInGlobal ? blob + (size_t)d.x * 128 : p),
-                            w, d.y, lane, shift);
+                            w, d.y, far.out, lane, shift);
             return true;
         default:
-            return slice<1>(a, p, w, far, d.y, m, uni, lane, shift, pol_stream, status);
+            return slice<1, COLLECT>(a, p, w, far, d.y, m, uni, lane, shift, pol_stream, status);
     }
 }
 

@@ -35,12 +35,20 @@ struct UnitTable {
     int numSlices = 0;
     const int4 *slice = nullptr;  // blob offset / 128, n, m | uniform << 8, bytes to stage / 128
     const char *blob = nullptr;
+    bool regular = false;  // at least half of the stencils are in uniform slices
+    int numStencils = 0;
 };
 
-// Tables from this size on get the layout beside the sliced one: below it there are too few slices
-// for the SMs' warps (8-wide level-3 rows, against the sliced layout: 131 k stencils 10.3 and 10.3
-// us, 295 k 12.3 and 14.7 us, 524 k 18.0 and 20.7 us, 1.2 M 26.5 and 39.0 us).
-constexpr int kUnitTable = 262144;
+// Tables from kUnitTable stencils on get the layout beside the sliced one.  A batch takes it for all
+// of them: its jobs together fill the SMs.  A single call takes it from kUnitCall on; below, there
+// are too few slices for the SMs' warps (8-wide level-3 rows, against the sliced layout: 131 k
+// stencils 10.3 and 10.3 us, 295 k 12.3 and 14.7 us, 524 k 14.8 and 20.7 us, 1.2 M 29.1 and 39.0 us).
+// Output rows that are not 16-byte aligned are collected, which costs about a third more
+// instructions: a single call takes the layout for them from kUnitAnyRow on, and for regular tables
+// only (5-wide rows: level 3 of quads, 1.2 M stencils 41.5 and 45.2 us, 2.1 M 59.7 and 71.8 us; level
+// 4 of triangles split at random, 1.2 M 50.1 and 39.7 us; in a batch, where the other jobs hide
+// what such a table waits for, they are taken with the rest: 464 and 469 us for the scene).
+constexpr int kUnitTable = 1 << 16, kUnitCall = 1 << 18, kUnitAnyRow = 3 << 19;
 
 constexpr int kUnitMost = 16;  // stencils per unit
 constexpr int kUnitList = 16;  // entries held in registers
@@ -57,12 +65,10 @@ int build_units(int numStencils, const int *sizes, const int *offsets, const int
                 const float *weights, cudaStream_t s, UnitTable &t, void *owned[2],
                 const char *who);
 
-// Whether the layout's kernels take these rows: both 16-byte aligned, strides multiples of 4
-// floats.  They write a stencil's row by itself (its neighbours in the output belong to other
-// units), which costs a row of 12 bytes as many 32-byte sectors as it has elements: over a table of
-// 2.1 M level-3 stencils rows of 8 floats take 39.6 us, of 3 floats 51.7 us and of 5 floats 75.0 us,
-// where the sliced layout (sell.h), which writes rows in table order, takes 64.3, 53.4 and 71.8 us.
-bool units_take(const float *src, int srcStride, const float *dst, int dstStride);
+// Whether the layout's kernels read these source rows: 16-byte aligned, the stride a multiple of 4
+// floats.  Output rows may have any layout; those that are not 16-byte aligned are collected.
+bool units_take(const float *src, int srcStride);
+bool units_collect(const float *dst, int dstStride);
 
 int eval_stencils_units(const UnitTable &t, const float *src, float *dst, int dstStride,
                         int length, int srcStride, cudaStream_t s, const char *who);

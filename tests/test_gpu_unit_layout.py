@@ -121,3 +121,40 @@ def test_infinite_control_point_and_batch(tables):
         for j, p in zip(jobs, plain):
             assert torch.equal(torch.nan_to_num(j[3]), torch.nan_to_num(p))
     assert batch.GetDeviceStatus() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length,stride,out_stride", [(3, 3, 3), (5, 5, 5), (3, 4, 5), (7, 8, 7),
+                                                      (11, 11, 11), (20, 20, 21)])
+def test_unaligned_output_rows(length, stride, out_stride):
+    """Output rows that no vector store takes (collected before they are written): a batch of tables
+    above and below the layout's size, and a single call on a regular table large enough for it."""
+    torch = torch_cuda()
+    from opensubdiv_gb300.evaluator import BufferDescriptor as BD, GB300Evaluator as Ev
+    from opensubdiv_gb300.evaluator import GB300StencilBatch, GB300StencilTable
+    rng = np.random.default_rng(length)
+    jobs, want = [], []
+    for n in (65535, 65536, 100003):
+        t = _table(n, n + length)
+        src = rng.uniform(-1, 1, NCV * stride).astype(np.float32)
+        out = torch.zeros(n * out_stride, device="cuda")
+        jobs.append((GB300StencilTable.Create(*t), dev(src), BD(0, length, stride), out,
+                     BD(0, length, out_stride)))
+        want.append((src, (0, length, stride), (0, length, out_stride), n, t))
+    GB300StencilBatch(jobs).Eval()
+    torch.cuda.synchronize()
+    for j, w in zip(jobs, want):
+        _check(host(j[3]).reshape(-1), *w)
+    # 98304 groups of 16 stencils with the same weights: 1.5 M stencils
+    n, k = 3 << 19, 7
+    first = rng.integers(0, NCV - k, n // 16)
+    idx = (np.repeat(first, 16)[:, None] + np.arange(k)).astype(np.int32).ravel()
+    w = np.tile(rng.uniform(-0.2, 1.0, (16, k)).astype(np.float32), (n // 16, 1)).ravel()
+    t = (np.full(n, k, np.int32), (np.arange(n) * k).astype(np.int32), idx, w)
+    table = GB300StencilTable.Create(*t)
+    src = rng.uniform(-1, 1, NCV * stride).astype(np.float32)
+    out = torch.zeros(n * out_stride, device="cuda")
+    assert Ev.EvalStencilsTable(dev(src), BD(0, length, stride), out, BD(0, length, out_stride),
+                                table)
+    Ev.Synchronize()
+    _check(host(out).reshape(-1), src, (0, length, stride), (0, length, out_stride), n, t)
