@@ -45,6 +45,32 @@ void scratch_free(void *p, cudaStream_t s);
 // GB300GetDeviceStatus reads and clears; staged kernels record an expired bounded wait there).
 int status_word_address(int **out);
 
+// Launches `kern` as the programmatic dependent of the kernel queued before it: it may be started
+// while that one still runs (at once if it called launch_dependents, else when it ends), and calls
+// wait_for_primary before it touches anything that work queued earlier reads or writes.  What it may
+// read before is a table's own layout, whose builder synchronised before it returned the table.
+// A captured launch keeps its plain dependency on whatever node precedes it.
+template <class K, class A>
+void launch_kernel(K kern, int grid, int threads, size_t smem, cudaStream_t s, const A &arg) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+        cudaGetLastError();
+        cs = cudaStreamCaptureStatusActive;
+    }
+    c.attrs = &attr;
+    c.numAttrs = cs == cudaStreamCaptureStatusNone ? 1 : 0;
+    cudaLaunchKernelEx(&c, kern, arg);  // the caller checks the launch
+    count_launch();
+}
+
 // Runs `fn` (returning a status) once per device for one call site: `done` is that call site's
 // bitmask of devices it already succeeded on (devices >= 64 run it every time).
 template <class F>
@@ -59,6 +85,16 @@ int once_per_device(std::atomic<uint64_t> &done, F fn) {
 }
 
 // ---- device helpers -----------------------------------------------------------------------
+
+// Programmatic dependent launch (launch_kernel).  launch_dependents lets the next kernel be started
+// as soon as every CTA of this one runs; it is then resident, and waits in wait_for_primary until
+// this one is done and its writes are visible.
+__device__ __forceinline__ void launch_dependents() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_primary() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // L2 eviction policies (createpolicy) for the cache-hinted loads below.
 __device__ __forceinline__ uint64_t l2_evict_first() {

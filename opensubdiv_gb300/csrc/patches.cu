@@ -106,6 +106,8 @@ __device__ __forceinline__ void store_packed(float *dst, float *stage, const flo
 template <int LC, int ORDER, bool QUAD = false, bool V4 = false>
 __global__ void __launch_bounds__(128, LC == 4 ? 4 : (ORDER < 2 && !V4 ? (QUAD ? 7 : 6) : 5))
     k_eval_patches(const PatchArgs a) {
+    launch_dependents();
+    wait_for_primary();
     constexpr bool PACK = LC > 1 && (!QUAD || V4);
     const int stride = gridDim.x * blockDim.x;
     if constexpr (!PACK) {
@@ -165,6 +167,8 @@ __global__ void __launch_bounds__(128, LC == 4 ? 4 : (ORDER < 2 && !V4 ? (QUAD ?
 // group (cheap for the separable quad-family bases this kernel is used for).
 template <int G, int ORDER>
 __global__ void __launch_bounds__(256, 4) k_eval_patches_lanes(const PatchArgs a) {
+    launch_dependents();
+    wait_for_primary();
     // G need not be a power of two: a warp holds floor(32 / G) groups (3 lanes per point
     // for xyz: 10 points per warp) and its remaining lanes stay idle
     constexpr int kPerWarp = 32 / G;
@@ -208,13 +212,13 @@ __global__ void __launch_bounds__(256, 4) k_eval_patches_lanes(const PatchArgs a
 template <int ORDER>
 void launch_lanes(int G, int grid, int threads, cudaStream_t s, const PatchArgs &a) {
     switch (G) {
-        case 1: k_eval_patches_lanes<1, ORDER><<<grid, threads, 0, s>>>(a); break;
-        case 2: k_eval_patches_lanes<2, ORDER><<<grid, threads, 0, s>>>(a); break;
-        case 3: k_eval_patches_lanes<3, ORDER><<<grid, threads, 0, s>>>(a); break;
-        case 4: k_eval_patches_lanes<4, ORDER><<<grid, threads, 0, s>>>(a); break;
-        case 6: k_eval_patches_lanes<6, ORDER><<<grid, threads, 0, s>>>(a); break;
-        case 8: k_eval_patches_lanes<8, ORDER><<<grid, threads, 0, s>>>(a); break;
-        default: k_eval_patches_lanes<32, ORDER><<<grid, threads, 0, s>>>(a); break;
+        case 1: launch_kernel(k_eval_patches_lanes<1, ORDER>, grid, threads, 0, s, a); break;
+        case 2: launch_kernel(k_eval_patches_lanes<2, ORDER>, grid, threads, 0, s, a); break;
+        case 3: launch_kernel(k_eval_patches_lanes<3, ORDER>, grid, threads, 0, s, a); break;
+        case 4: launch_kernel(k_eval_patches_lanes<4, ORDER>, grid, threads, 0, s, a); break;
+        case 6: launch_kernel(k_eval_patches_lanes<6, ORDER>, grid, threads, 0, s, a); break;
+        case 8: launch_kernel(k_eval_patches_lanes<8, ORDER>, grid, threads, 0, s, a); break;
+        default: launch_kernel(k_eval_patches_lanes<32, ORDER>, grid, threads, 0, s, a); break;
     }
 }
 
@@ -224,15 +228,15 @@ void launch_points(int length, int grid, int threads, cudaStream_t s, const Patc
     const bool v4 = ((uintptr_t)a.src & 15) == 0 && a.srcStride % 4 == 0 &&
                     (a.length % 4 == 0 || a.quadRows);
     switch (length) {
-        case 1: k_eval_patches<1, ORDER, QUAD><<<grid, threads, 0, s>>>(a); break;
-        case 2: k_eval_patches<2, ORDER, QUAD><<<grid, threads, 0, s>>>(a); break;
+        case 1: launch_kernel(k_eval_patches<1, ORDER, QUAD>, grid, threads, 0, s, a); break;
+        case 2: launch_kernel(k_eval_patches<2, ORDER, QUAD>, grid, threads, 0, s, a); break;
         case 3:
-            if (v4) k_eval_patches<3, ORDER, QUAD, true><<<grid, threads, 0, s>>>(a);
-            else k_eval_patches<3, ORDER, QUAD><<<grid, threads, 0, s>>>(a);
+            if (v4) launch_kernel(k_eval_patches<3, ORDER, QUAD, true>, grid, threads, 0, s, a);
+            else launch_kernel(k_eval_patches<3, ORDER, QUAD>, grid, threads, 0, s, a);
             break;
         default:
-            if (v4) k_eval_patches<4, ORDER, QUAD, true><<<grid, threads, 0, s>>>(a);
-            else k_eval_patches<4, ORDER, QUAD><<<grid, threads, 0, s>>>(a);
+            if (v4) launch_kernel(k_eval_patches<4, ORDER, QUAD, true>, grid, threads, 0, s, a);
+            else launch_kernel(k_eval_patches<4, ORDER, QUAD>, grid, threads, 0, s, a);
             break;
     }
 }
@@ -281,7 +285,6 @@ int eval_patches(const float *src, float *const *dst, const int *strides, int le
         if (order == 0) launch_lanes<0>(G, grid, threads, s, a);
         else if (order == 1) launch_lanes<1>(G, grid, threads, s, a);
         else launch_lanes<2>(G, grid, threads, s, a);
-        count_launch();
         return check_launch(who);
     }
     // one thread per point: tables with triangle patches, and points grouped by patch (a
@@ -300,7 +303,6 @@ int eval_patches(const float *src, float *const *dst, const int *strides, int le
         else if (order == 1) launch_points<1, false>(length, grid, threads, s, a);
         else launch_points<2, false>(length, grid, threads, s, a);
     }
-    count_launch();
     return check_launch(who);
 }
 

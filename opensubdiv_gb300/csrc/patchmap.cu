@@ -136,6 +136,8 @@ struct FindArgs {
 // handles computed from the leaf; of a triangle tree 74.8 us, 37.5 us with both and the sums
 // compared without the FP64 pipe (patchmap_walk.cuh).
 __global__ void __launch_bounds__(256) k_find_patches(const FindArgs a) {
+    launch_dependents();
+    wait_for_primary();
     __shared__ int stage[8][32 * 5];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int stride = gridDim.x * blockDim.x;
@@ -190,8 +192,7 @@ int find_patches(const PatchMapDevice &m, int n, const int *faces, const float *
     const int threads = 256;
     long long blocks = ((long long)n + threads - 1) / threads;
     long long cap = (long long)num_sms() * 16;
-    k_find_patches<<<(int)(blocks < cap ? blocks : cap), threads, 0, s>>>(a);
-    count_launch();
+    launch_kernel(k_find_patches, (int)(blocks < cap ? blocks : cap), threads, 0, s, a);
     return check_launch("FindPatches");
 }
 

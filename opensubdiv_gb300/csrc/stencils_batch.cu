@@ -557,6 +557,8 @@ __global__ void __launch_bounds__(256) k_pad_rows(const PadJob *jobs, const long
 }
 
 __global__ void __launch_bounds__(256) k_pad_one(const PadJob j) {
+    launch_dependents();
+    wait_for_primary();
     const long long step = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < j.numRows;
          i += step)
@@ -567,8 +569,7 @@ int launch_pad_one(const PadJob &j, cudaStream_t s) {
     if (j.numRows <= 0) return GB300_OK;
     const long long blocks = (j.numRows + 255) / 256;
     const int grid = (int)std::min<long long>(blocks, (long long)num_sms() * 16);
-    k_pad_one<<<grid, 256, 0, s>>>(j);
-    count_launch();
+    launch_kernel(k_pad_one, grid, 256, 0, s, j);
     return check_launch("padded source copy");
 }
 

@@ -377,6 +377,7 @@ __device__ __forceinline__ void store_cols(const SellArgs &a, int o, int row, in
 template <int NW, int VW>
 __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow) ? 3 : NW >= 6 && VW != kNarrow ? 1 : 2)
     k_stencils_sell(const SellArgs a) {
+    launch_dependents();
     extern __shared__ __align__(128) char smem[];
     using C = SellCfg<NW, VW>;
     constexpr int S = C::kRing, SPT = C::kSpt;
@@ -442,6 +443,8 @@ __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow
     // slice wg of the tile
     const int grp = warp / GW, wg = warp - grp * GW;
     if (grp >= G) return;
+    // the producer streams the table, which no queued work writes, while the kernel before ends
+    wait_for_primary();
     // entry steps gathered together, columns per pass
     constexpr int R = VW == kNarrow ? (NW == 1 ? 6 : 4) : VW == 12 ? 2 : NW <= 3 ? 4 : 2;
     constexpr int CW = VW == 12 ? 12 : VW == kNarrow ? 4 : 8;
@@ -549,8 +552,7 @@ static int launch_sell(const SellArgs &a, cudaStream_t s) {
     SellArgs b = a;
     b.numTiles = (a.numSlices + C::kSpt - 1) / C::kSpt;
     const int grid = min(b.numTiles, num_sms() * perSm);
-    kern<<<grid, kThreads, C::kSmem, s>>>(b);
-    count_launch();
+    launch_kernel(kern, grid, kThreads, C::kSmem, s, b);
     return GB300_OK;
 }
 

@@ -21,6 +21,7 @@ struct Args {
 
 template <bool COLLECT>
 __global__ void __launch_bounds__(kThreads, 1) k_stencils_units(const Args a) {
+    launch_dependents();
     extern __shared__ __align__(128) char smem[];
     __shared__ Queue queue[kWarps];
     __shared__ int claimed;
@@ -47,11 +48,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_stencils_units(const Args a) {
     claim();
     Feed f;
     Far far = warp_far(bytes, q.far);
+    bool wait = true;  // for the kernel before; the table's slices are on their way meanwhile
     for (;; ++f.popped) {
         while (more && f.room(q, d.w)) {
             f.push(q, bytes, a.blob, d, lane, pol_stream);
             claim();
         }
+        if (wait) wait_for_primary();
+        wait = false;
         if (f.popped == f.pushed) return;
         const int s = f.popped % kAhead;
         if (!ring::wait(&q.full[s], (uint32_t)(f.popped / kAhead) & 1, a.status)) return;
@@ -106,8 +110,8 @@ int eval_stencils_units(const UnitTable &t, const float *src, float *dst, int ds
     a.numSlices = t.numSlices;
     a.dst[0] = dst;
     a.dstStride[0] = dstStride;
-    kern<<<min(a.numSlices, num_sms()), units::kThreads, units::kSmemBytes, s>>>(a);
-    count_launch();
+    launch_kernel(kern, min(a.numSlices, num_sms()), units::kThreads, units::kSmemBytes, s,
+                  a);
     return check_launch(who);
 }
 
