@@ -50,10 +50,10 @@ int status_word_address(int **out);
 // wait_for_primary before it touches anything that work queued earlier reads or writes.  What it may
 // read before is a table's own layout, whose builder synchronised before it returned the table.
 // A captured launch keeps its plain dependency on whatever node precedes it.
-template <class K, class A>
-void launch_kernel(K kern, int grid, int threads, size_t smem, cudaStream_t s, const A &arg) {
+template <class K, class... A>
+void launch_kernel(K kern, dim3 grid, int threads, size_t smem, cudaStream_t s, const A &... arg) {
     cudaLaunchConfig_t c = {};
-    c.gridDim = dim3((unsigned)grid);
+    c.gridDim = grid;
     c.blockDim = dim3((unsigned)threads);
     c.dynamicSmemBytes = smem;
     c.stream = s;
@@ -67,7 +67,7 @@ void launch_kernel(K kern, int grid, int threads, size_t smem, cudaStream_t s, c
     }
     c.attrs = &attr;
     c.numAttrs = cs == cudaStreamCaptureStatusNone ? 1 : 0;
-    cudaLaunchKernelEx(&c, kern, arg);  // the caller checks the launch
+    cudaLaunchKernelEx(&c, kern, arg...);  // the caller checks the launch
     count_launch();
 }
 

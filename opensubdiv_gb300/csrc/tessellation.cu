@@ -139,6 +139,10 @@ struct GenArgs {
     int *owners;
     int *faceSlot;
     unsigned int slotMask;
+    // the patterns to generate: the slots of the table in use, and -1 - f for a face f without
+    // one; *listed is their number less one
+    int *list;
+    int *listed;
 };
 
 __device__ __forceinline__ bool uses_shared(const GenArgs &a, int N) {
@@ -214,6 +218,7 @@ __device__ __forceinline__ unsigned int key_hash(unsigned long long k) {
 // Neighbouring faces often share a key, so the lanes of a warp with the same key insert once,
 // through their lowest lane (the lowest face of the group).
 __global__ void __launch_bounds__(256) k_tess_dedupe(const GenArgs a) {
+    launch_dependents();
     const int stride = gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
     // every lane runs the same number of iterations, so the warp stays converged
@@ -231,17 +236,26 @@ __global__ void __launch_bounds__(256) k_tess_dedupe(const GenArgs a) {
         const unsigned same = __match_any_sync(0xffffffffu, key) & keyedMask;
         const int leader = same ? __ffs(same) - 1 : lane;
         int slot = -1;
+        bool fresh = f < a.numFaces && !keyed;  // a new entry of the list
         if (keyed && leader == lane) {
             unsigned int h = key_hash(key) & a.slotMask;
             for (unsigned int probe = 0; probe <= a.slotMask; ++probe) {
                 const unsigned long long prev = atomicCAS(a.keys + h, kEmptyKey, key);
                 if (prev == kEmptyKey || prev == key) {
+                    fresh = prev == kEmptyKey;
                     atomicMin(a.owners + h, f);
                     slot = (int)h;
                     break;
                 }
                 h = (h + 1) & a.slotMask;
             }
+        }
+        const unsigned entries = __ballot_sync(0xffffffffu, fresh);
+        if (entries) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(a.listed, __popc(entries)) + 1;
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(entries & ((1u << lane) - 1));
+            if (fresh) a.list[at] = keyed ? slot : -1 - f;
         }
         slot = __shfl_sync(0xffffffffu, slot, leader);
         if (f < a.numFaces) a.faceSlot[f] = keyed ? slot : -1;
@@ -255,42 +269,65 @@ __device__ __forceinline__ int owner_of(const GenArgs &a, int f) {
     return slot < 0 ? f : a.owners[slot];
 }
 
-// One thread per face without a shared pattern: the face's coords or its facets (indices already
-// offset to the mesh numbering) straight into its slice of the output, for the faces of
+// One thread's part of a face without a shared pattern: runs of its coords or strips of its facets
+// (indices already offset to the mesh numbering) straight into its slice of the output, for faces of
 // parameterization kind K.
 template <int K, bool COORDS>
-__device__ __forceinline__ void generate_faces(const GenArgs &a) {
-    const int stride = gridDim.x * blockDim.x;
-    for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < a.numFaces; f += stride) {
-        const int N = a.faceSizes[f];
-        const int kind = N == a.reg ? (a.reg == 4 ? tess::kQuad : tess::kTri) : tess::kQsub;
-        if (kind != K || uses_shared(a, N) || owner_of(a, f) != f) continue;
-        FaceRates r;
-        rates_of(a.rateOffsets, a.rates, a.uniformRate, f, r);
-        Face face;
-        if (!face.init(a.reg, N, r.n, r.p, a.fs, a.pq, r.one)) continue;
-        const int64_t c0 = a.co[f];
-        Sink o{a.coords + c0 * a.coordStride, a.coordStride, a.facets + a.fo[f] * a.facetStride,
-               a.fs, a.facetStride, a.offsetIndices ? (int)c0 : 0, a.coordPairs != 0};
-        if constexpr (COORDS) face.coords_k<K>(o);
-        else face.facets_k<K>(o);
+__device__ __forceinline__ void generate_face(const GenArgs &a, int f, int part, int parts) {
+    const int N = a.faceSizes[f];
+    const int kind = N == a.reg ? (a.reg == 4 ? tess::kQuad : tess::kTri) : tess::kQsub;
+    if (kind != K || uses_shared(a, N)) return;
+    FaceRates r;
+    rates_of(a.rateOffsets, a.rates, a.uniformRate, f, r);
+    Face face;
+    if (!face.init(a.reg, N, r.n, r.p, a.fs, a.pq, r.one)) return;
+    const int64_t c0 = a.co[f];
+    Sink o{a.coords + c0 * a.coordStride, a.coordStride, a.facets + a.fo[f] * a.facetStride,
+           a.fs, a.facetStride, a.offsetIndices ? (int)c0 : 0, a.coordPairs != 0, part, parts};
+    if constexpr (COORDS) face.coords_k<K>(o);
+    else face.facets_k<K>(o);
+}
+
+constexpr int kRows = 8;  // rows of blocks per kind of work, if there is a list
+
+template <int K, bool COORDS>
+__device__ __forceinline__ void generate_faces(const GenArgs &a, int row) {
+    const int thread = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+    if (!a.dedupe) {
+        for (int f = thread; f < a.numFaces; f += threads) generate_face<K, COORDS>(a, f, 0, 1);
+        return;
+    }
+    // the rows share each pattern's runs and strips while that leaves every thread one pattern at
+    // most, and the patterns otherwise
+    const int count = *a.listed + 1;
+    int parts = kRows;
+    while (parts > 1 && count > threads * (kRows / parts)) parts >>= 1;
+    for (int64_t x = thread + (int64_t)(row / parts) * threads; x < count;
+         x += (int64_t)threads * (kRows / parts)) {
+        const int e = a.list[x];
+        generate_face<K, COORDS>(a, e < 0 ? -1 - e : a.owners[e], row & (parts - 1), parts);
     }
 }
 
-// Blocks of row y of the grid generate part `first` + y.  A mesh has few distinct patterns, so the
-// launch lasts as long as one thread takes for its longest part: the parts -- two kinds of face,
-// coords and facets -- run at the same time, in one launch (a launch per kind, each thread coords and facets:
-// 41 + 23 us for the per-edge rates of 69 k faces; now 37 us).  Each block's code is one part's.
+// Rows of blocks generate work `first` + y / rows.  A mesh has few distinct patterns, so the launch
+// lasts as long as one thread takes for its longest share: a pattern's coords and facets, of
+// either kind of face, run at the same time, and so do its runs and strips, each
+// row of blocks its own, so that the lanes of a warp do the same runs of different patterns (per-edge
+// rates of 69 k faces: 41 + 23 us with a launch per kind and one thread per pattern, 37 us with
+// coords and facets apart, 20 us so).
 constexpr int kQuadParts = 0, kQsubParts = 2, kTriParts = 4;
 
 __global__ void __launch_bounds__(128, 8) k_tess_generate(const GenArgs a, int first) {
-    switch (first + (int)blockIdx.y) {
-        case kQuadParts: generate_faces<tess::kQuad, false>(a); break;
-        case kQuadParts + 1: generate_faces<tess::kQuad, true>(a); break;
-        case kQsubParts: generate_faces<tess::kQsub, false>(a); break;
-        case kQsubParts + 1: generate_faces<tess::kQsub, true>(a); break;
-        case kTriParts: generate_faces<tess::kTri, false>(a); break;
-        default: generate_faces<tess::kTri, true>(a); break;
+    launch_dependents();
+    wait_for_primary();
+    const int row = a.dedupe ? (int)blockIdx.y % kRows : 0;
+    switch (first + (int)blockIdx.y / (a.dedupe ? kRows : 1)) {
+        case kQuadParts: generate_faces<tess::kQuad, false>(a, row); break;
+        case kQuadParts + 1: generate_faces<tess::kQuad, true>(a, row); break;
+        case kQsubParts: generate_faces<tess::kQsub, false>(a, row); break;
+        case kQsubParts + 1: generate_faces<tess::kQsub, true>(a, row); break;
+        case kTriParts: generate_faces<tess::kTri, false>(a, row); break;
+        default: generate_faces<tess::kTri, true>(a, row); break;
     }
 }
 
@@ -316,9 +353,16 @@ __device__ __forceinline__ void move_facets(const GenArgs &a, const int *from, i
                                             int nf, int delta, int lane) {
     int *to = a.facets + f0 * a.facetStride;
     if (a.facetStride == FS && step == FS) {
-        for (int q = lane; q < nf * FS; q += 32) {
-            const int v = from[q];
-            to[q] = v >= 0 ? v + delta : v;
+        // four loads in flight per lane: the slices may have left L2 (7 k copied faces of 500
+        // facets: 108 us with one, 53 us so)
+        constexpr int U = 4;
+        for (int q = lane; q < nf * FS; q += 32 * U) {
+            int v[U];
+#pragma unroll
+            for (int m = 0; m < U; ++m) v[m] = q + 32 * m < nf * FS ? from[q + 32 * m] : 0;
+#pragma unroll
+            for (int m = 0; m < U; ++m)
+                if (q + 32 * m < nf * FS) to[q + 32 * m] = v[m] >= 0 ? v[m] + delta : v[m];
         }
         return;
     }
@@ -337,6 +381,8 @@ __device__ __forceinline__ void move_facets(const GenArgs &a, const int *from, i
 // into its own (coords as float2 pairs), and locates every coord of the face on the patch table.
 template <int FS>
 __global__ void __launch_bounds__(256) k_tess_finish(const GenArgs a) {
+    launch_dependents();
+    wait_for_primary();
     __shared__ int stages[8][160];
     const int lane = threadIdx.x & 31;
     int *stage = stages[threadIdx.x >> 5];
@@ -1054,13 +1100,15 @@ extern "C" int GB300TessellationGenerate(
         while (cap < 2u * (unsigned int)numFaces && cap < (1u << 30)) cap <<= 1;
         const size_t kb = sizeof(unsigned long long) * cap, ob = sizeof(int) * cap;
         const size_t fb = sizeof(int) * (size_t)numFaces;
-        st = scratch_alloc(&dd, kb + ob + fb, s, who);
+        st = scratch_alloc(&dd, kb + 16 + ob + 2 * fb, s, who);
         if (st == GB300_OK) {
             a.keys = (unsigned long long *)dd;
-            a.owners = (int *)((char *)dd + kb);
-            a.faceSlot = (int *)((char *)dd + kb + ob);
+            a.listed = (int *)((char *)dd + kb);
+            a.owners = (int *)((char *)dd + kb + 16);
+            a.faceSlot = (int *)((char *)dd + kb + 16 + ob);
+            a.list = (int *)((char *)dd + kb + 16 + ob + fb);
             a.slotMask = cap - 1;
-            st = check_cuda(cudaMemsetAsync(a.keys, 0xff, kb, s), who);
+            st = check_cuda(cudaMemsetAsync(a.keys, 0xff, kb + 16, s), who);  // and *listed: -1
             if (st == GB300_OK) st = check_cuda(cudaMemsetAsync(a.owners, 0x7f, ob, s), who);
         }
         if (st == GB300_OK) {
@@ -1073,22 +1121,25 @@ extern "C" int GB300TessellationGenerate(
     if (st == GB300_OK) {
         // with shared patterns only polygons above 10 sides are generated per face: none for
         // a triangle scheme, only quad sub-face polygons for a quad scheme
-        const int grid = grid_for(numFaces, 128, 16);
+        const int wide = grid_for(numFaces, 128, 16);
         if (regularFaceSize == 4 || !a.shared) {
             const int first = regularFaceSize == 3 ? kTriParts : a.shared ? kQsubParts : kQuadParts;
             const int parts = regularFaceSize == 4 && !a.shared ? 4 : 2;
-            k_tess_generate<<<dim3(grid, parts), 128, 0, s>>>(a, first);
-            count_launch();
+            // with a list, as many blocks in all rows together as are resident (8 per SM), and as
+            // many as give each face a thread, should each have its own pattern
+            const int rows = a.dedupe ? kRows : 1;
+            const int grid = std::min(wide, std::max(8 * num_sms() / (rows * parts),
+                                                     (wide + rows - 1) / rows));
+            launch_kernel(k_tess_generate, dim3(grid, parts * rows), 128, 0, s, a, first);
         }
         st = check_launch(who);
     }
     if (st == GB300_OK && (a.shared || a.locate || a.dedupe)) {
         const int blocks = grid_for((long long)numFaces * 32, 256, 8);
         if (o.fs == 4)
-            k_tess_finish<4><<<blocks, 256, 0, s>>>(a);
+            launch_kernel(k_tess_finish<4>, blocks, 256, 0, s, a);
         else
-            k_tess_finish<3><<<blocks, 256, 0, s>>>(a);
-        count_launch();
+            launch_kernel(k_tess_finish<3>, blocks, 256, 0, s, a);
         st = check_launch(who);
     }
     if (dd) scratch_free(dd, s);
