@@ -538,7 +538,11 @@ int GB300PatchTableEval(const GB300PatchTable *t, const float *src, float *dst, 
     cudaStream_t s = as_stream(stream);
     // Loop tables are evaluated one point per thread, 13 rows each: rows of 3 floats are read from
     // a copy padded to 4 (one load per row), as soon as there are more points than rows to copy
-    // (4 M points, 226 k rows: 298 us, and 238 + 4 us with the copy).  Catmull-Clark tables read a
+    // (4 M points, 226 k rows: 298 us, and 238 + 4 us with the copy).  With derivatives and as many
+    // points as patch indices the copy has a row per index, so that a patch's rows follow one another
+    // and no index is read (4 M points, copy included: six outputs 250 -> 220 us over 1.0 M indices
+    // and 271 -> 256 over 4.1 M, P and the first derivatives 230 -> 186; P alone 94.5 -> 95.4 of
+    // 2 M points: not there).  Catmull-Clark tables read a
     // row with 3 lanes in one access; a padded copy costs them more than it saves (332 us, and
     // 366 + 24 us over 5.7 M rows).  Not while the stream is captured: the copy's memory would
     // become part of the caller's graph.
@@ -547,13 +551,17 @@ int GB300PatchTableEval(const GB300PatchTable *t, const float *src, float *dst, 
         numPatchCoords >= 65536 && numPatchCoords >= t->numControl && t->numControl > 0 &&
         cudaStreamIsCapturing(s, &capture) == cudaSuccess &&
         capture == cudaStreamCaptureStatusNone) {
+        const bool gather = (du || dv || duu || duv || dvv) && t->numIndices <= numPatchCoords;
+        const size_t rows = gather ? (size_t)t->numIndices : (size_t)t->numControl;
         float *padded = nullptr;
-        if (scratch_alloc((void **)&padded, (size_t)t->numControl * 16, s, who) == GB300_OK) {
+        if (scratch_alloc((void **)&padded, rows * 16, s, who) == GB300_OK) {
+            const int *indices = (const int *)t->indices;
             batch::PadJob j{src, padded, srcStride, length, t->numControl, 4, 0};
-            int r = batch::launch_pad_one(j, s);
+            int r = gather ? gather_patch_rows(src, srcStride, indices, (int)rows, padded, s)
+                           : batch::launch_pad_one(j, s);
             if (r == GB300_OK)
                 r = eval_patches(padded, d, st, length, 4, numPatchCoords, patchCoords, t->arrays,
-                                 (const int *)t->indices, t->params, s, who, 0, 0, 1);
+                                 indices, t->params, s, who, 0, 0, gather ? 2 : 1);
             scratch_free(padded, s);
             return r != GB300_OK ? r : check_launch(who);
         }

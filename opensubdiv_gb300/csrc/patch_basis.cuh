@@ -51,10 +51,19 @@ struct Acc6 {
 // query that lands on the same patch: they are loaded with an evict-last L2 policy, so the
 // streams read or written once (query coords, outputs) do not push them out of L2.
 
-// Loads LC elements [e0, e0+LC) of control point `cv` (elements >= length read as 0).  V4: rows of
-// 3 or 4 elements whose 16 bytes are aligned (and inside the row's stride): one load per row;
-// elements >= length are whatever the row's stride holds, and are not written.
-template <int LC, bool V4>
+// How the source rows lie (V4): kAnyRows; kQuadRows, rows of 3 or 4 elements whose 16 bytes are
+// aligned (and inside the row's stride); kPatchRows, quads in the order of the patch's own control
+// points, from src on, so that no index is read.
+enum SourceRows { kAnyRows = 0, kQuadRows = 1, kPatchRows = 2 };
+
+template <int V4>
+__device__ __forceinline__ int row_index(const int *__restrict__ cvs, int j) {
+    return V4 == kPatchRows ? j : __ldg(cvs + j);
+}
+
+// Loads LC elements [e0, e0+LC) of control point `cv` (elements >= length read as 0): quads in one
+// load, whose elements >= length are whatever the row's stride holds, and are not written.
+template <int LC, int V4>
 __device__ __forceinline__ void load_row(const float *__restrict__ src, int stride, int cv,
                                          int e0, int length, float (&x)[LC]) {
     const float *p = src + (size_t)cv * stride + e0;
@@ -79,7 +88,7 @@ __device__ __forceinline__ void load_row(const float *__restrict__ src, int stri
 // then scale with the patch's extent instead of the points' distance from the origin, and
 // the float rounding of the cancelling derivative sums (which carry the 2^depth and 4^depth
 // factors) shrinks by that ratio.  The value output adds xc back at the end.
-template <int LC, bool V4>
+template <int LC, int V4>
 __device__ __forceinline__ void load_row(const float *__restrict__ src, int stride, int cv,
                                          int e0, int length, float (&x)[LC],
                                          const float (&xc)[LC]) {
@@ -103,8 +112,13 @@ __device__ __forceinline__ void add_origin(const float (&xc)[LC], Acc6<LC> &acc)
 
 // N control-point indices of a patch: 128-bit loads when the index row is 16-byte aligned
 // (REGULAR rows are 64 B, GREGORY_BASIS rows 80 B), scalar loads otherwise.
-template <int N>
+template <int N, int V4>
 __device__ __forceinline__ void load_indices(const int *__restrict__ cvs, int (&idx)[N]) {
+    if constexpr (V4 == kPatchRows) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) idx[j] = j;
+        return;
+    }
     const uint64_t pol = l2_evict_last();
     if ((N % 4) == 0 && (reinterpret_cast<uintptr_t>(cvs) & 15) == 0) {
 #pragma unroll
@@ -182,7 +196,7 @@ __device__ __forceinline__ void tensor_accumulate(const float (&sp)[4], const fl
 }
 
 // REGULAR: 16 points in row-major (t rows, s columns) order.
-template <int LC, bool V4 = false>
+template <int LC, int V4 = 0>
 __device__ void eval_bspline(float s, float t, int boundary, const int *__restrict__ cvs,
                              const float *__restrict__ src, int stride, int e0, int length,
                              Acc6<LC> &acc) {
@@ -195,7 +209,7 @@ __device__ void eval_bspline(float s, float t, int boundary, const int *__restri
     if (boundary & 4) { fold_last(tp); fold_last(td); fold_last(tdd); }
     if (boundary & 8) { fold_first(sp); fold_first(sd); fold_first(sdd); }
     int idx[16];
-    load_indices<16>(cvs, idx);
+    load_indices<16, V4>(cvs, idx);
     float xc[LC];  // point 5: the patch's (0,0) corner, never a phantom
     if constexpr (LC == 1) {  // all 16 rows in flight at a time
         float x[16][1];
@@ -226,7 +240,7 @@ __device__ void eval_bspline(float s, float t, int boundary, const int *__restri
 // GREGORY_BASIS: 20 points; the Bezier grid is
 //   row 0: 0 1 7 5 | row 1: 2 (3,4) (8,9) 6 | row 2: 16 (18,19) (13,14) 12 | row 3: 15 17 11 10
 // where (a,b) is the pair of interior face points blended by G (patchBasis.h:346-378).
-template <int LC, bool V4 = false>
+template <int LC, int V4 = 0>
 __device__ void eval_gregory(float s, float t, const int *__restrict__ cvs,
                              const float *__restrict__ src, int stride, int e0, int length,
                              Acc6<LC> &acc) {
@@ -240,7 +254,7 @@ __device__ void eval_gregory(float s, float t, const int *__restrict__ cvs,
     float d3 = s + tc;  d3 = (d3 <= 0.0f) ? 1.0f : (1.0f / d3);
     const float g0 = s * d0, g2 = t * d1, g4 = sc * d2, g6 = tc * d3;
     int idx[20];
-    load_indices<20>(cvs, idx);
+    load_indices<20, V4>(cvs, idx);
     float xc[LC];  // point 0: the patch's (0,0) corner
     load_row<LC, V4>(src, stride, idx[0], e0, length, xc);
     // rows of the Bezier grid; interior entries are blended pairs
@@ -324,7 +338,7 @@ __device__ __forceinline__ void bezier_tri_weights(float u, float v, int ds, int
 
 // GREGORY_TRIANGLE: 18 points mapped onto the 15 quartic Bezier points; interior Bezier
 // points 6, 7 and 10 are blends of Gregory pairs (3,4), (8,9), (13,14) (patchBasis.h:1078-1106).
-template <int LC, bool V4 = false>
+template <int LC, int V4 = 0>
 __device__ void eval_gregory_tri(float s, float t, const int *__restrict__ cvs,
                                  const float *__restrict__ src, int stride, int e0, int length,
                                  Acc6<LC> &acc) {
@@ -336,20 +350,20 @@ __device__ void eval_gregory_tri(float s, float t, const int *__restrict__ cvs,
     // Bezier point m comes from Gregory point kBez[m] (or a blended pair for 6, 7, 10)
     constexpr int kBez[15] = {0, 1, 15, 7, 5, 2, -1, -2, 6, 17, -3, 16, 11, 12, 10};
     float xc[LC];  // point 0: the (0,0) corner
-    load_row<LC, V4>(src, stride, __ldg(cvs), e0, length, xc);
+    load_row<LC, V4>(src, stride, row_index<V4>(cvs, 0), e0, length, xc);
     float B[15][LC];
 #pragma unroll
     for (int m = 0; m < 15; ++m) {
         const int gi = kBez[m];
         if (gi >= 0) {
-            load_row<LC, V4>(src, stride, __ldg(cvs + gi), e0, length, B[m], xc);
+            load_row<LC, V4>(src, stride, row_index<V4>(cvs, gi), e0, length, B[m], xc);
         } else {
             const int a = (gi == -1) ? 3 : (gi == -2) ? 8 : 13;
             const float ga = (gi == -1) ? g[0] : (gi == -2) ? g[2] : g[4];
             const float gb = (gi == -1) ? g[1] : (gi == -2) ? g[3] : g[5];
             float xa[LC], xb[LC];
-            load_row<LC, V4>(src, stride, __ldg(cvs + a), e0, length, xa, xc);
-            load_row<LC, V4>(src, stride, __ldg(cvs + a + 1), e0, length, xb, xc);
+            load_row<LC, V4>(src, stride, row_index<V4>(cvs, a), e0, length, xa, xc);
+            load_row<LC, V4>(src, stride, row_index<V4>(cvs, a + 1), e0, length, xb, xc);
 #pragma unroll
             for (int c = 0; c < LC; ++c) B[m][c] = ga * xa[c] + gb * xb[c];
         }
@@ -469,7 +483,7 @@ __device__ __forceinline__ void box_weights(int k, const float *m, float (&w)[12
     }
 }
 
-template <int LC, bool V4 = false>
+template <int LC, int V4 = 0>
 __device__ void eval_box_tri(float s, float t, int boundary, const int *__restrict__ cvs,
                              const float *__restrict__ src, int stride, int e0, int length,
                              Acc6<LC> &acc) {
@@ -484,7 +498,7 @@ __device__ void eval_box_tri(float s, float t, int boundary, const int *__restri
     float x[12][LC], xc[LC];
     {
         int idx[12];
-        load_indices<12>(cvs, idx);
+        load_indices<12, V4>(cvs, idx);
         load_row<LC, V4>(src, stride, idx[4], e0, length, xc);  // point 4: the (0,0) corner
 #pragma unroll
         for (int j = 0; j < 12; ++j) load_row<LC, V4>(src, stride, idx[j], e0, length, x[j], xc);
@@ -504,7 +518,7 @@ __device__ void eval_box_tri(float s, float t, int boundary, const int *__restri
     add_origin<LC>(xc, acc);
 }
 
-template <int LC, bool V4 = false>
+template <int LC, int V4 = 0>
 __device__ void eval_linear_quad(float s, float t, const int *__restrict__ cvs,
                                  const float *__restrict__ src, int stride, int e0, int length,
                                  Acc6<LC> &acc) {
@@ -514,11 +528,11 @@ __device__ void eval_linear_quad(float s, float t, const int *__restrict__ cvs,
     const float wt[4] = {-sc, -s, s, sc};
     const float wst[4] = {1.0f, -1.0f, 1.0f, -1.0f};
     float xc[LC];
-    load_row<LC, V4>(src, stride, __ldg(cvs), e0, length, xc);
+    load_row<LC, V4>(src, stride, row_index<V4>(cvs, 0), e0, length, xc);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         float x[LC];
-        load_row<LC, V4>(src, stride, __ldg(cvs + j), e0, length, x, xc);
+        load_row<LC, V4>(src, stride, row_index<V4>(cvs, j), e0, length, x, xc);
 #pragma unroll
         for (int c = 0; c < LC; ++c) {
             acc.v[0][c] = fmaf(wp[j], x[c], acc.v[0][c]);
@@ -530,14 +544,14 @@ __device__ void eval_linear_quad(float s, float t, const int *__restrict__ cvs,
     add_origin<LC>(xc, acc);
 }
 
-template <int LC, bool V4 = false>
+template <int LC, int V4 = 0>
 __device__ void eval_linear_tri(float s, float t, const int *__restrict__ cvs,
                                 const float *__restrict__ src, int stride, int e0, int length,
                                 Acc6<LC> &acc) {
     float x0[LC], x1[LC], x2[LC];
-    load_row<LC, V4>(src, stride, __ldg(cvs + 0), e0, length, x0);
-    load_row<LC, V4>(src, stride, __ldg(cvs + 1), e0, length, x1, x0);
-    load_row<LC, V4>(src, stride, __ldg(cvs + 2), e0, length, x2, x0);
+    load_row<LC, V4>(src, stride, row_index<V4>(cvs, 0), e0, length, x0);
+    load_row<LC, V4>(src, stride, row_index<V4>(cvs, 1), e0, length, x1, x0);
+    load_row<LC, V4>(src, stride, row_index<V4>(cvs, 2), e0, length, x2, x0);
     // relative to point 0: P = x0 + s (x1 - x0) + t (x2 - x0)
 #pragma unroll
     for (int c = 0; c < LC; ++c) {
@@ -550,7 +564,7 @@ __device__ void eval_linear_tri(float s, float t, const int *__restrict__ cvs,
 // OsdEvaluatePatchBasis + gather for one point: normalises (s,t) into the patch, evaluates
 // the basis of `type`, accumulates into acc and returns the derivative scales d1, d2
 // (patchBasis.h:1558-1610).  Returns false for an unknown type.
-template <int LC, bool QUAD_ONLY = false, bool V4 = false>
+template <int LC, bool QUAD_ONLY = false, int V4 = 0>
 __device__ bool eval_patch_point(int type, Param p, float s, float t,
                                  const int *__restrict__ cvs, const float *__restrict__ src,
                                  int stride, int e0, int length, Acc6<LC> &acc, float &d1,

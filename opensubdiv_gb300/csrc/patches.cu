@@ -50,7 +50,7 @@ struct PatchArgs {
     const Array *arrays;
     const int *indices;
     const ParamRec *params;
-    int quadRows;  // source rows are padded to quads
+    int rows;  // kQuadRows: source rows are padded to quads; kPatchRows: and one per patch index
 };
 
 // Highest output index a derivative order needs: 0 P only, 1 P + du + dv, 2 all six.  The
@@ -58,7 +58,7 @@ struct PatchArgs {
 __host__ __device__ constexpr int last_output(int order) { return order == 0 ? 0 : order == 1 ? 2 : 5; }
 
 // Elements [e0, e0 + LC) of all outputs of the point at c, and the outputs' scales.
-template <int LC, bool QUAD, bool V4>
+template <int LC, bool QUAD, int V4>
 __device__ __forceinline__ void eval_point(const PatchArgs &a, const Coord &c, int e0,
                                            Acc6<LC> &acc, float (&scale)[6]) {
     acc.zero();
@@ -68,10 +68,10 @@ __device__ __forceinline__ void eval_point(const PatchArgs &a, const Coord &c, i
         const ParamRec pr = load_param(a.params + c.patchIndex);
         const Param p{pr.field0, pr.field1};
         const int type = p.regular() ? arr.regDesc : arr.desc;
-        const int *cvs =
-            a.indices + arr.indexBase + arr.stride * (c.patchIndex - arr.primitiveIdBase);
-        if (!eval_patch_point<LC, QUAD, V4>(type, p, c.s, c.t, cvs, a.src, a.srcStride, e0,
-                                            a.length, acc, d1, d2))
+        const int first = arr.indexBase + arr.stride * (c.patchIndex - arr.primitiveIdBase);
+        const float *src = V4 == kPatchRows ? a.src + (size_t)first * 4 : a.src;
+        if (!eval_patch_point<LC, QUAD, V4>(type, p, c.s, c.t, a.indices + first, src,
+                                            a.srcStride, e0, a.length, acc, d1, d2))
             acc.zero();
     }
     scale[0] = 1.0f;
@@ -102,8 +102,9 @@ __device__ __forceinline__ void store_packed(float *dst, float *stage, const flo
 // QUAD: Catmull-Clark tables (REGULAR / GREGORY_BASIS / QUADS only): without the Loop and
 // triangle bases the kernel fits 7 blocks per SM for orders 0 and 1 without spills; it is bound by
 // instruction issue (61%), and the packed stores cost it more (79 -> 87 us for 1.7 M coords).
-// V4: source rows are read as one quad each (patch_basis.cuh).
-template <int LC, int ORDER, bool QUAD = false, bool V4 = false>
+// V4: source rows are read as one quad each (patch_basis.cuh; with a row per patch index 4 M Loop
+// points of six outputs take 220 us, copy included, with a row per control point 250).
+template <int LC, int ORDER, bool QUAD = false, int V4 = kAnyRows>
 __global__ void __launch_bounds__(128, LC == 4 ? 4 : (ORDER < 2 && !V4 ? (QUAD ? 7 : 6) : 5))
     k_eval_patches(const PatchArgs a) {
     launch_dependents();
@@ -226,25 +227,63 @@ template <int ORDER, bool QUAD>
 void launch_points(int length, int grid, int threads, cudaStream_t s, const PatchArgs &a) {
     // whole quads at 16-byte aligned addresses: nothing past a row's elements is read
     const bool v4 = ((uintptr_t)a.src & 15) == 0 && a.srcStride % 4 == 0 &&
-                    (a.length % 4 == 0 || a.quadRows);
+                    (a.length % 4 == 0 || a.rows);
     switch (length) {
         case 1: launch_kernel(k_eval_patches<1, ORDER, QUAD>, grid, threads, 0, s, a); break;
         case 2: launch_kernel(k_eval_patches<2, ORDER, QUAD>, grid, threads, 0, s, a); break;
         case 3:
-            if (v4) launch_kernel(k_eval_patches<3, ORDER, QUAD, true>, grid, threads, 0, s, a);
+            if constexpr (!QUAD) {
+                if (a.rows == kPatchRows) {
+                    launch_kernel(k_eval_patches<3, ORDER, false, kPatchRows>, grid, threads, 0, s, a);
+                    break;
+                }
+            }
+            if (v4) launch_kernel(k_eval_patches<3, ORDER, QUAD, kQuadRows>, grid, threads, 0, s, a);
             else launch_kernel(k_eval_patches<3, ORDER, QUAD>, grid, threads, 0, s, a);
             break;
         default:
-            if (v4) launch_kernel(k_eval_patches<4, ORDER, QUAD, true>, grid, threads, 0, s, a);
+            if (v4) launch_kernel(k_eval_patches<4, ORDER, QUAD, kQuadRows>, grid, threads, 0, s, a);
             else launch_kernel(k_eval_patches<4, ORDER, QUAD>, grid, threads, 0, s, a);
             break;
     }
 }
 
+// One quad per patch index: the row of 3 floats that it names.
+struct GatherArgs {
+    const float *src;
+    int srcStride;
+    const int *indices;
+    int n;
+    float4 *rows;
+};
+
+__global__ void __launch_bounds__(256) k_gather_patch_rows(const GatherArgs a) {
+    launch_dependents();
+    wait_for_primary();
+    const int stride = gridDim.x * blockDim.x;
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < a.n; j += stride) {
+        const int cv = __ldg(a.indices + j);
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (cv >= 0) {
+            const float *p = a.src + (size_t)cv * a.srcStride;
+            v.x = __ldg(p), v.y = __ldg(p + 1), v.z = __ldg(p + 2);
+        }
+        a.rows[j] = v;
+    }
+}
+
+int gather_patch_rows(const float *src, int srcStride, const int *indices, int n, float *rows,
+                      cudaStream_t s) {
+    const GatherArgs a{src, srcStride, indices, n, reinterpret_cast<float4 *>(rows)};
+    const int blocks = (n + 255) / 256, cap = num_sms() * 8;
+    launch_kernel(k_gather_patch_rows, blocks < cap ? blocks : cap, 256, 0, s, a);
+    return GB300_OK;
+}
+
 int eval_patches(const float *src, float *const *dst, const int *strides, int length,
                  int srcStride, int numCoords, const void *coords, const void *arrays,
                  const int *indices, const void *params, cudaStream_t s, const char *who,
-                 int quadFamily, int grouped, int quadRows) {
+                 int quadFamily, int grouped, int rows) {
     if (numCoords <= 0) return ok();
     if (!src || !coords || !arrays || !indices || !params)
         return fail(GB300_ERR_INVALID_ARGUMENT, "%s: null source, coord or table pointer", who);
@@ -260,7 +299,7 @@ int eval_patches(const float *src, float *const *dst, const int *strides, int le
     a.arrays = (const Array *)arrays;
     a.indices = indices;
     a.params = (const ParamRec *)params;
-    a.quadRows = quadRows;
+    a.rows = rows;
     for (int k = 0; k < 6; ++k) {
         if (!dst[k]) continue;
         if (strides[k] < length)

@@ -53,11 +53,16 @@ int eval_stencils(const float *src, float *const *dst, const int *strides,
 // selects the element-lane kernel (known for device tables; raw-pointer calls pass 0).
 // grouped: consecutive coords mostly share a patch (a tessellation's coords), which selects
 // the one-thread-per-point kernel for every table.
-// quadRows: the source rows are a copy padded to whole quads, which may be read whole.
+// rows: kQuadRows (1), the source rows are a copy padded to whole quads, which may be read whole;
+// kPatchRows (2), and that copy has one row per entry of `indices` (gather_patch_rows).
 int eval_patches(const float *src, float *const *dst, const int *strides, int length,
                  int srcStride, int numCoords, const void *coords, const void *arrays,
                  const int *indices, const void *params, cudaStream_t s, const char *who,
-                 int quadFamily, int grouped = 0, int quadRows = 0);
+                 int quadFamily, int grouped = 0, int rows = 0);
+
+// rows[j] = the 3 floats of source row indices[j], j < n, as quads.
+int gather_patch_rows(const float *src, int srcStride, const int *indices, int n, float *rows,
+                      cudaStream_t s);
 
 // Draw-time tessellation factors of every patch of a table (tess_factors.cu).
 int tess_factors(const void *arrays, int numArrays, const int *indices, const void *params,

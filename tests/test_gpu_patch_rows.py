@@ -1,5 +1,5 @@
 """EvalPatches over the source and output layouts that choose a kernel: Loop tables with more points
-than source rows (a copy padded to quads), rows of whole quads, packed outputs (written through shared
+than source rows (a copy padded to quads), or than patch indices (a copy of a row per index), rows of whole quads, packed outputs (written through shared
 memory, whole sectors at a time) and outputs inside wider rows, at point counts around a warp and
 around the padded copy's threshold.  Accuracy gate of tests/gpu_util.py (1e-5 x the bounding-box
 diagonal against the oracle, second derivatives against its FP64 form)."""
@@ -20,7 +20,7 @@ GOLDEN = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden")
 @pytest.mark.parametrize("points,length,stride,out_stride,outputs", [
     (1, 3, 3, 3, 6), (31, 4, 4, 4, 3), (33, 4, 8, 4, 6), (257, 8, 8, 8, 6), (65535, 3, 3, 3, 3),
     (65536, 3, 3, 3, 6), (65569, 3, 3, 4, 6), (65537, 3, 4, 3, 1), (66001, 3, 5, 3, 3)])
-def test_rows_and_counts(table, points, length, stride, out_stride, outputs):
+def test_rows_and_counts(table, points, length, stride, out_stride, outputs, more=0):
     torch = torch_cuda()
     from opensubdiv_gb300.evaluator import (BufferDescriptor as BD, GB300Evaluator as Ev,
                                             GB300PatchTable)
@@ -30,7 +30,8 @@ def test_rows_and_counts(table, points, length, stride, out_stride, outputs):
     rows[:, :length] = (smooth_primvars(xyz)[:, :length] if length > 3 else xyz)
     rows[:, length:] = np.nan  # what a wider row holds must not reach the result
     coords = z["coords"][np.arange(points) % len(z["coords"])]
-    t = GB300PatchTable.Create(z["arrays"], z["patch_indices"], z["params"],
+    indices = np.concatenate([z["patch_indices"], np.zeros(more, np.int32)])
+    t = GB300PatchTable.Create(z["arrays"], indices, z["params"],
                                triangular=bool(z["triangular"]))
     out = [torch.full((points * out_stride,), 7.0, device="cuda") for _ in range(outputs)]
     d, kw = BD(0, length, out_stride), {}
@@ -51,3 +52,10 @@ def test_rows_and_counts(table, points, length, stride, out_stride, outputs):
         got = host(out[k]).reshape(points, out_stride)
         gate(f"{table} rows", k, got[:, :length].ravel(), ref[0][k], ref[1][k], diag)
         assert (got[:, length:] == 7.0).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("outputs", [1, 3, 6])
+def test_more_indices_than_points(outputs):
+    """More points than source rows, but not than patch indices (the last ones unused)."""
+    test_rows_and_counts("icosphere2_patches_L3", 65536, 3, 3, 3, outputs, more=65536)
