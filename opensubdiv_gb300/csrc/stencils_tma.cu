@@ -20,7 +20,8 @@
 // Table objects evaluate through their sliced layout (sell.h) with k_stencils_sell: the same
 // producer / ring / consumer-group scheme, tiles of whole 32-stencil slices, one consumer warp
 // per slice stepping through entry j of its 32 stencils together (one conflict-free 32-bit
-// shared load per array per step).  The Far-layout kernel serves raw-pointer calls.
+// shared load per array per step); large tables of one output through their unit layout
+// (stencils_units.cu).  The Far-layout kernel serves raw-pointer calls.
 #include "common.cuh"
 #include "sell.h"
 #include "stencil_eval.cuh"
