@@ -49,6 +49,10 @@ int status_word_address(int **out);
 // while that one still runs (at once if it called launch_dependents, else when it ends), and calls
 // wait_for_primary before it touches anything that work queued earlier reads or writes.  What it may
 // read before is a table's own layout, whose builder synchronised before it returned the table.
+// Anything else is written during the lifetime of such a kernel, as far as the memory model goes,
+// so it is read with coherent loads, which the wait orders: the ones below, or C++ loads through
+// pointers that are not __restrict__.  The non-coherent path (ld.global.nc, __ldg) is for the
+// tables' own arrays.
 // A captured launch keeps its plain dependency on whatever node precedes it.
 template <class K, class... A>
 void launch_kernel(K kern, dim3 grid, int threads, size_t smem, cudaStream_t s, const A &... arg) {
@@ -95,6 +99,11 @@ __device__ __forceinline__ void launch_dependents() {
 __device__ __forceinline__ void wait_for_primary() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// The pointer as it stands behind the wait: a load through it depends on this, and so on the wait.
+template <class T>
+__device__ __forceinline__ void behind_wait(T *&p) {
+    asm volatile("" : "+l"(p) : : "memory");
+}
 
 // L2 eviction policies (createpolicy) for the cache-hinted loads below.
 __device__ __forceinline__ uint64_t l2_evict_first() {
@@ -109,7 +118,8 @@ __device__ __forceinline__ uint64_t l2_evict_last() {
 }
 
 // Streaming (read-once) 32-bit loads for the stencil table: no L1 allocation and an
-// evict-first L2 policy, so the table stream does not push the source rows out of L2.
+// evict-first L2 policy, so the table stream does not push the source rows out of L2.  Non-coherent:
+// for a table's own arrays, or in kernels that are launched behind all earlier work.
 __device__ __forceinline__ int ld_stream(const int *p, uint64_t pol) {
     int v;
     asm("ld.global.nc.L1::no_allocate.L2::cache_hint.b32 %0, [%1], %2;"
@@ -123,25 +133,63 @@ __device__ __forceinline__ float ld_stream(const float *p, uint64_t pol) {
     return v;
 }
 
-// Source-row loads: read-only path, kept in L1, evict-last in L2 (the control points are
-// re-read by every stencil that touches them).
+// Coherent loads of the caller's data, which a kernel queued before may write.  Two forms keep them
+// behind wait_for_primary: the volatile ones stand where the program has them, among themselves and
+// against the wait; the others the compiler may move, as far as their address allows, which is to
+// come from behind_wait.  (EvalPatches, 4 M points: lanes with volatile rows and indices 374 -> 396
+// us, their loads no longer overlapping as the compiler had them; Loop rows through behind_wait 255
+// -> 261 us, for the registers of the pointer.)
+//
+// Source rows: kept in L1, evict-last in L2 (the control points are re-read by every stencil that
+// touches them).
 __device__ __forceinline__ float ld_src(const float *p, uint64_t pol) {
     float v;
-    asm("ld.global.nc.L1::evict_last.L2::cache_hint.f32 %0, [%1], %2;"
-                 : "=f"(v) : "l"(p), "l"(pol));
+    asm("ld.global.L1::evict_last.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
     return v;
 }
-
+__device__ __forceinline__ float4 ld_src4(const float *p) {
+    float4 v;
+    asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_row4(const float *p, uint64_t pol) {
+    float4 v;
+    asm volatile("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p), "l"(pol)
+                 : "memory");
+    return v;
+}
+// Indices of patches.
 __device__ __forceinline__ int ld_keep(const int *p, uint64_t pol) {
     int v;
-    asm("ld.global.nc.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+    asm("ld.global.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
     return v;
 }
 __device__ __forceinline__ int4 ld_keep4(const int *p, uint64_t pol) {
     int4 v;
-    asm("ld.global.nc.L2::cache_hint.v4.b32 {%0, %1, %2, %3}, [%4], %5;"
+    asm("ld.global.L2::cache_hint.v4.b32 {%0, %1, %2, %3}, [%4], %5;"
         : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
         : "l"(p), "l"(pol));
+    return v;
+}
+// Params of patches, and queries (read once: no L1 allocation).
+__device__ __forceinline__ int ld_param(const int *p, uint64_t pol) {
+    int v;
+    asm volatile("ld.global.L2::cache_hint.b32 %0, [%1], %2;"
+                 : "=r"(v)
+                 : "l"(p), "l"(pol)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ int ld_query(const int *p, uint64_t pol) {
+    int v;
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.b32 %0, [%1], %2;"
+                 : "=r"(v)
+                 : "l"(p), "l"(pol)
+                 : "memory");
     return v;
 }
 

@@ -57,24 +57,24 @@ struct Acc6 {
 enum SourceRows { kAnyRows = 0, kQuadRows = 1, kPatchRows = 2 };
 
 template <int V4>
-__device__ __forceinline__ int row_index(const int *__restrict__ cvs, int j) {
-    return V4 == kPatchRows ? j : __ldg(cvs + j);
+__device__ __forceinline__ int row_index(const int *cvs, int j) {
+    return V4 == kPatchRows ? j : ld_keep(cvs + j, l2_evict_last());
 }
 
 // Loads LC elements [e0, e0+LC) of control point `cv` (elements >= length read as 0): quads in one
 // load, whose elements >= length are whatever the row's stride holds, and are not written.
 template <int LC, int V4>
-__device__ __forceinline__ void load_row(const float *__restrict__ src, int stride, int cv,
+__device__ __forceinline__ void load_row(const float *src, int stride, int cv,
                                          int e0, int length, float (&x)[LC]) {
     const float *p = src + (size_t)cv * stride + e0;
     const uint64_t pol = l2_evict_last();
     if constexpr (V4) {
         static_assert(LC == 3 || LC == 4, "one quad per row");
-        const int4 v = ld_keep4(reinterpret_cast<const int *>(p), pol);
-        x[0] = __int_as_float(v.x);
-        x[1] = __int_as_float(v.y);
-        x[2] = __int_as_float(v.z);
-        if constexpr (LC == 4) x[3] = __int_as_float(v.w);
+        const float4 v = ld_row4(p, pol);
+        x[0] = v.x;
+        x[1] = v.y;
+        x[2] = v.z;
+        if constexpr (LC == 4) x[3] = v.w;
     } else {
 #pragma unroll
         for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? ld_src(p + c, pol) : 0.0f;
@@ -89,7 +89,7 @@ __device__ __forceinline__ void load_row(const float *__restrict__ src, int stri
 // the float rounding of the cancelling derivative sums (which carry the 2^depth and 4^depth
 // factors) shrinks by that ratio.  The value output adds xc back at the end.
 template <int LC, int V4>
-__device__ __forceinline__ void load_row(const float *__restrict__ src, int stride, int cv,
+__device__ __forceinline__ void load_row(const float *src, int stride, int cv,
                                          int e0, int length, float (&x)[LC],
                                          const float (&xc)[LC]) {
     if constexpr (V4) {
@@ -113,7 +113,7 @@ __device__ __forceinline__ void add_origin(const float (&xc)[LC], Acc6<LC> &acc)
 // N control-point indices of a patch: 128-bit loads when the index row is 16-byte aligned
 // (REGULAR rows are 64 B, GREGORY_BASIS rows 80 B), scalar loads otherwise.
 template <int N, int V4>
-__device__ __forceinline__ void load_indices(const int *__restrict__ cvs, int (&idx)[N]) {
+__device__ __forceinline__ void load_indices(const int *cvs, int (&idx)[N]) {
     if constexpr (V4 == kPatchRows) {
 #pragma unroll
         for (int j = 0; j < N; ++j) idx[j] = j;
@@ -197,8 +197,8 @@ __device__ __forceinline__ void tensor_accumulate(const float (&sp)[4], const fl
 
 // REGULAR: 16 points in row-major (t rows, s columns) order.
 template <int LC, int V4 = 0>
-__device__ void eval_bspline(float s, float t, int boundary, const int *__restrict__ cvs,
-                             const float *__restrict__ src, int stride, int e0, int length,
+__device__ void eval_bspline(float s, float t, int boundary, const int *cvs,
+                             const float *src, int stride, int e0, int length,
                              Acc6<LC> &acc) {
     float sp[4], sd[4], sdd[4], tp[4], td[4], tdd[4];
     bspline_curve(s, sp, sd, sdd);
@@ -241,8 +241,8 @@ __device__ void eval_bspline(float s, float t, int boundary, const int *__restri
 //   row 0: 0 1 7 5 | row 1: 2 (3,4) (8,9) 6 | row 2: 16 (18,19) (13,14) 12 | row 3: 15 17 11 10
 // where (a,b) is the pair of interior face points blended by G (patchBasis.h:346-378).
 template <int LC, int V4 = 0>
-__device__ void eval_gregory(float s, float t, const int *__restrict__ cvs,
-                             const float *__restrict__ src, int stride, int e0, int length,
+__device__ void eval_gregory(float s, float t, const int *cvs,
+                             const float *src, int stride, int e0, int length,
                              Acc6<LC> &acc) {
     float bs[4], bds[4], bdss[4], bt[4], bdt[4], bdtt[4];
     bezier_curve(s, bs, bds, bdss);
@@ -339,8 +339,8 @@ __device__ __forceinline__ void bezier_tri_weights(float u, float v, int ds, int
 // GREGORY_TRIANGLE: 18 points mapped onto the 15 quartic Bezier points; interior Bezier
 // points 6, 7 and 10 are blends of Gregory pairs (3,4), (8,9), (13,14) (patchBasis.h:1078-1106).
 template <int LC, int V4 = 0>
-__device__ void eval_gregory_tri(float s, float t, const int *__restrict__ cvs,
-                                 const float *__restrict__ src, int stride, int e0, int length,
+__device__ void eval_gregory_tri(float s, float t, const int *cvs,
+                                 const float *src, int stride, int e0, int length,
                                  Acc6<LC> &acc) {
     float g[6] = {1.0f, 0.0f, 1.0f, 0.0f, 1.0f, 0.0f};
     const float u = s, v = t, w = 1.0f - u - v;
@@ -484,8 +484,8 @@ __device__ __forceinline__ void box_weights(int k, const float *m, float (&w)[12
 }
 
 template <int LC, int V4 = 0>
-__device__ void eval_box_tri(float s, float t, int boundary, const int *__restrict__ cvs,
-                             const float *__restrict__ src, int stride, int e0, int length,
+__device__ void eval_box_tri(float s, float t, int boundary, const int *cvs,
+                             const float *src, int stride, int e0, int length,
                              Acc6<LC> &acc) {
     float m[15];
     m[0] = 1.0f; m[1] = s; m[2] = t;
@@ -519,8 +519,8 @@ __device__ void eval_box_tri(float s, float t, int boundary, const int *__restri
 }
 
 template <int LC, int V4 = 0>
-__device__ void eval_linear_quad(float s, float t, const int *__restrict__ cvs,
-                                 const float *__restrict__ src, int stride, int e0, int length,
+__device__ void eval_linear_quad(float s, float t, const int *cvs,
+                                 const float *src, int stride, int e0, int length,
                                  Acc6<LC> &acc) {
     const float sc = 1.0f - s, tc = 1.0f - t;
     const float wp[4] = {sc * tc, s * tc, s * t, sc * t};
@@ -545,8 +545,8 @@ __device__ void eval_linear_quad(float s, float t, const int *__restrict__ cvs,
 }
 
 template <int LC, int V4 = 0>
-__device__ void eval_linear_tri(float s, float t, const int *__restrict__ cvs,
-                                const float *__restrict__ src, int stride, int e0, int length,
+__device__ void eval_linear_tri(float s, float t, const int *cvs,
+                                const float *src, int stride, int e0, int length,
                                 Acc6<LC> &acc) {
     float x0[LC], x1[LC], x2[LC];
     load_row<LC, V4>(src, stride, row_index<V4>(cvs, 0), e0, length, x0);
@@ -566,7 +566,7 @@ __device__ void eval_linear_tri(float s, float t, const int *__restrict__ cvs,
 // (patchBasis.h:1558-1610).  Returns false for an unknown type.
 template <int LC, bool QUAD_ONLY = false, int V4 = 0>
 __device__ bool eval_patch_point(int type, Param p, float s, float t,
-                                 const int *__restrict__ cvs, const float *__restrict__ src,
+                                 const int *cvs, const float *src,
                                  int stride, int e0, int length, Acc6<LC> &acc, float &d1,
                                  float &d2) {
     const int depth = p.depth();

@@ -25,17 +25,17 @@ __device__ __forceinline__ Coord load_coord(const Coord *p) {
     const int *q = reinterpret_cast<const int *>(p);
     const uint64_t pol = l2_evict_first();
     Coord c;
-    c.arrayIndex = ld_stream(q, pol);
-    c.patchIndex = ld_stream(q + 1, pol);
-    c.vertIndex = ld_stream(q + 2, pol);
-    c.s = __int_as_float(ld_stream(q + 3, pol));
-    c.t = __int_as_float(ld_stream(q + 4, pol));
+    c.arrayIndex = ld_query(q, pol);
+    c.patchIndex = ld_query(q + 1, pol);
+    c.vertIndex = ld_query(q + 2, pol);
+    c.s = __int_as_float(ld_query(q + 3, pol));
+    c.t = __int_as_float(ld_query(q + 4, pol));
     return c;
 }
 __device__ __forceinline__ ParamRec load_param(const ParamRec *p) {
     const int *q = reinterpret_cast<const int *>(p);
     const uint64_t pol = l2_evict_last();
-    return ParamRec{ld_keep(q, pol), ld_keep(q + 1, pol), __int_as_float(ld_keep(q + 2, pol))};
+    return ParamRec{ld_param(q, pol), ld_param(q + 1, pol), __int_as_float(ld_param(q + 2, pol))};
 }
 
 struct PatchArgs {
@@ -52,6 +52,15 @@ struct PatchArgs {
     const ParamRec *params;
     int rows;  // kQuadRows: source rows are padded to quads; kPatchRows: and one per patch index
 };
+
+// The arguments with the pointers whose loads may move as they stand behind the wait.
+template <int V4>
+__device__ __forceinline__ PatchArgs args_behind_wait(const PatchArgs &arg) {
+    PatchArgs a = arg;
+    if (V4 == kAnyRows) behind_wait(a.src);
+    if (V4 != kPatchRows) behind_wait(a.indices);
+    return a;
+}
 
 // Highest output index a derivative order needs: 0 P only, 1 P + du + dv, 2 all six.  The
 // kernels are instantiated per order so the unused accumulations compile away.
@@ -106,9 +115,10 @@ __device__ __forceinline__ void store_packed(float *dst, float *stage, const flo
 // points of six outputs take 220 us, copy included, with a row per control point 250).
 template <int LC, int ORDER, bool QUAD = false, int V4 = kAnyRows>
 __global__ void __launch_bounds__(128, LC == 4 ? 4 : (ORDER < 2 && !V4 ? (QUAD ? 7 : 6) : 5))
-    k_eval_patches(const PatchArgs a) {
+    k_eval_patches(const PatchArgs arg) {
     launch_dependents();
     wait_for_primary();
+    const PatchArgs a = args_behind_wait<V4>(arg);
     constexpr bool PACK = LC > 1 && (!QUAD || V4);
     const int stride = gridDim.x * blockDim.x;
     if constexpr (!PACK) {
@@ -167,9 +177,10 @@ __global__ void __launch_bounds__(128, LC == 4 ? 4 : (ORDER < 2 && !V4 ? (QUAD ?
 // lane) and no cross-lane reduction is needed.  The basis is evaluated by every lane of the
 // group (cheap for the separable quad-family bases this kernel is used for).
 template <int G, int ORDER>
-__global__ void __launch_bounds__(256, 4) k_eval_patches_lanes(const PatchArgs a) {
+__global__ void __launch_bounds__(256, 4) k_eval_patches_lanes(const PatchArgs arg) {
     launch_dependents();
     wait_for_primary();
+    const PatchArgs a = args_behind_wait<kAnyRows>(arg);
     // G need not be a power of two: a warp holds floor(32 / G) groups (3 lanes per point
     // for xyz: 10 points per warp) and its remaining lanes stay idle
     constexpr int kPerWarp = 32 / G;
@@ -262,11 +273,11 @@ __global__ void __launch_bounds__(256) k_gather_patch_rows(const GatherArgs a) {
     wait_for_primary();
     const int stride = gridDim.x * blockDim.x;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < a.n; j += stride) {
-        const int cv = __ldg(a.indices + j);
+        const int cv = a.indices[j];
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (cv >= 0) {
             const float *p = a.src + (size_t)cv * a.srcStride;
-            v.x = __ldg(p), v.y = __ldg(p + 1), v.z = __ldg(p + 2);
+            v.x = p[0], v.y = p[1], v.z = p[2];
         }
         a.rows[j] = v;
     }

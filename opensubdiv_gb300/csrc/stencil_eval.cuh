@@ -8,6 +8,8 @@
 namespace gb300 {
 namespace tma {
 
+// Source rows are read with coherent loads: kernels queued before may write them (launch_kernel).
+//
 // Elements [c0, c0 + 8) of source row `id` (zeros past the primvar length): one 256-bit load
 // for 32-byte aligned rows, two 128-bit loads for 16-byte aligned rows, else scalar loads.
 // VW = 0 picks the width at run time from a.vw (one code path for jobs of mixed layouts).
@@ -23,16 +25,15 @@ __device__ __forceinline__ void gather_row(const A &a, int id, int c0, uint64_t 
         else
             gather_row<1>(a, id, c0, pol_src, x);
     } else if constexpr (VW == 8) {
-        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-            : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]),
-              "=f"(x[6]), "=f"(x[7])
-            : "l"(row));
+        asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]),
+                       "=f"(x[6]), "=f"(x[7])
+                     : "l"(row));
     } else if constexpr (VW == 4) {
-        const float4 *r4 = reinterpret_cast<const float4 *>(row);
-        const float4 v0 = __ldg(r4);
+        const float4 v0 = ld_src4(row);
         x[0] = v0.x; x[1] = v0.y; x[2] = v0.z; x[3] = v0.w;
         if (c0 + 4 < a.length) {
-            const float4 v1 = __ldg(r4 + 1);
+            const float4 v1 = ld_src4(row + 4);
             x[4] = v1.x; x[5] = v1.y; x[6] = v1.z; x[7] = v1.w;
         } else {
             x[4] = x[5] = x[6] = x[7] = 0.0f;
@@ -157,11 +158,10 @@ __device__ __forceinline__ void eval_one12(const A &a, int i, int n, const int *
 #pragma unroll
             for (int m = 0; m < 2; ++m)
                 if (q + g + m >= o && q + g + m < end) {
-                    const float4 *r = reinterpret_cast<const float4 *>(
-                        a.src + (size_t)ids[g + m] * a.srcStride);
-                    x[m][0] = __ldg(r);
-                    x[m][1] = __ldg(r + 1);
-                    x[m][2] = __ldg(r + 2);
+                    const float *r = a.src + (size_t)ids[g + m] * a.srcStride;
+                    x[m][0] = ld_src4(r);
+                    x[m][1] = ld_src4(r + 4);
+                    x[m][2] = ld_src4(r + 8);
                 }
 #pragma unroll
             for (int m = 0; m < 2; ++m) {

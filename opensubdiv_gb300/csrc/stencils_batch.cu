@@ -533,7 +533,7 @@ __device__ __forceinline__ void pad_row(const PadJob &j, long long i) {
     for (int c0 = 0; c0 < j.dstStride; c0 += 4) {
         float x[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) x[c] = c0 + c < j.length ? __ldg(row + c0 + c) : 0.0f;
+        for (int c = 0; c < 4; ++c) x[c] = c0 + c < j.length ? row[c0 + c] : 0.0f;
         *reinterpret_cast<float4 *>(d + c0) = make_float4(x[0], x[1], x[2], x[3]);
     }
 }

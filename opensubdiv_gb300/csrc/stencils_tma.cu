@@ -310,6 +310,11 @@ struct SellArgs {
     unsigned magic;  // 65536 / length + 1
 };
 
+struct SourceRows {  // gather_row's view
+    const float *src;
+    int srcStride, length;
+};
+
 struct SellMeta {
     int s0, s1, slot0, staged;
 };
@@ -318,20 +323,19 @@ struct SellMeta {
 // 16-byte loads; the row stride is a multiple of 4 floats, at least 12), or the 4 columns of a
 // row of at most 4 floats (VW = kNarrow: one 16-byte load, stride a multiple of 4).
 template <int VW>
-__device__ __forceinline__ void gather_cols(const SellArgs &a, int id, int c0, uint64_t pol_src,
+__device__ __forceinline__ void gather_cols(const SourceRows &a, int id, int c0, uint64_t pol_src,
                                             float (&x)[VW == 12 ? 12 : VW == kNarrow ? 4 : 8]) {
     if constexpr (VW == kNarrow) {
-        const float4 q =
-            __ldg(reinterpret_cast<const float4 *>(a.src + (size_t)id * a.srcStride + c0));
+        const float4 q = ld_src4(a.src + (size_t)id * a.srcStride + c0);
         x[0] = q.x;
         x[1] = q.y;
         x[2] = q.z;
         x[3] = q.w;
     } else if constexpr (VW == 12) {
-        const float4 *r = reinterpret_cast<const float4 *>(a.src + (size_t)id * a.srcStride);
+        const float *r = a.src + (size_t)id * a.srcStride;
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
-            const float4 q = __ldg(r + v);
+            const float4 q = ld_src4(r + 4 * v);
             x[4 * v] = q.x;
             x[4 * v + 1] = q.y;
             x[4 * v + 2] = q.z;
@@ -446,6 +450,8 @@ __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow
     if (grp >= G) return;
     // the producer streams the table, which no queued work writes, while the kernel before ends
     wait_for_primary();
+    SourceRows rows{a.src, a.srcStride, a.length};
+    behind_wait(rows.src);
     // entry steps gathered together, columns per pass
     constexpr int R = VW == kNarrow ? (NW == 1 ? 6 : 4) : VW == 12 ? 2 : NW <= 3 ? 4 : 2;
     constexpr int CW = VW == 12 ? 12 : VW == kNarrow ? 4 : 8;
@@ -500,7 +506,7 @@ __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow
                     float x[R][CW];
 #pragma unroll
                     for (int q = 0; q < R; ++q)
-                        if (!SKIP || j0 + q < n) gather_cols<VW>(a, ids[q], c0, pol_src, x[q]);
+                        if (!SKIP || j0 + q < n) gather_cols<VW>(rows, ids[q], c0, pol_src, x[q]);
 #pragma unroll
                     for (int q = 0; q < R; ++q)
                         if (j0 + q < n)

@@ -20,7 +20,8 @@ struct Args {
 };
 
 template <bool COLLECT>
-__global__ void __launch_bounds__(kThreads, 1) k_stencils_units(const Args a) {
+__global__ void __launch_bounds__(kThreads, 1) k_stencils_units(const Args arg) {
+    Args a = arg;
     launch_dependents();
     extern __shared__ __align__(128) char smem[];
     __shared__ Queue queue[kWarps];
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_stencils_units(const Args a) {
             claim();
         }
         if (wait) wait_for_primary();
+        behind_wait(a.src);
         wait = false;
         if (f.popped == f.pushed) return;
         const int s = f.popped % kAhead;
