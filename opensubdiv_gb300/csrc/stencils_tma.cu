@@ -78,6 +78,51 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity) {
     }
     return true;
 }
+// A consumer group's wait for its tile `it` in a ring of S stages that G groups take turns on.  The
+// use of the stage is told by its parity, which tells it from the use before only if that one has
+// completed.  With S a multiple of G the group consumed that one itself.  Else it was another
+// group's and may still be on its way, copies of two stages completing in any order, when this group
+// is done with a tile of its own behind it: the parity would pass at once, for a stage that holds
+// neither tile.  So the producer numbers the stage's tile, once the use before is consumed, and
+// the group waits for the number first (8-wide rows, 3 stages and 2 groups: 20.4 and 20.5 us).
+template <int S, int G>
+struct Turns {
+    static constexpr bool kNumbered = S % G != 0;
+    int tile[kNumbered ? S : 1];
+    __device__ __forceinline__ void init() {
+        if (kNumbered)
+            for (int s = 0; s < S; ++s) tile[s] = -1;
+    }
+    // by one lane of the producer, behind its wait for the empty stage
+    __device__ __forceinline__ void number(int stage, int it) {
+        if (kNumbered)
+            asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tile + stage)),
+                         "r"(it)
+                         : "memory");
+    }
+    __device__ __forceinline__ bool is(int stage, int it) const {
+        int v;
+        asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];"
+                     : "=r"(v)
+                     : "r"(smem_u32(tile + stage))
+                     : "memory");
+        return v == it;
+    }
+    // Bounded, as mbar_wait.
+    __device__ __forceinline__ bool wait(uint64_t *full, int it) const {
+        const int stage = it % S;
+        if (kNumbered && !is(stage, it)) {
+            const unsigned long long t0 = now_ns();
+            while (!is(stage, it)) {
+                if (now_ns() - t0 > kWaitNs) {
+                    atomicExch(&g_status, GB300_ERR_DEVICE_TIMEOUT);
+                    return false;
+                }
+            }
+        }
+        return mbar_wait(&full[stage], (uint32_t)(it / S) & 1);
+    }
+};
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes,
                                          uint64_t *bar, uint64_t policy) {
     asm volatile(
@@ -137,6 +182,7 @@ __global__ void __launch_bounds__(kThreads, NW >= 6 ? 1 : 2) k_stencils_tma(cons
     constexpr int S = C::kRing;
     __shared__ __align__(8) uint64_t full[S], empty[S];
     __shared__ Meta meta[S];
+    __shared__ Turns<S, kConsumers / C::kTile> turns;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Consumer groups: a tile holds kTile stencils (one per thread), fewer than the consumers
     // when every stencil carries 3 or 6 weight arrays; the consumers then split into groups
@@ -151,6 +197,7 @@ __global__ void __launch_bounds__(kThreads, NW >= 6 ? 1 : 2) k_stencils_tma(cons
             mbar_init(&full[s], 32);
             mbar_init(&empty[s], GW);  // one group consumes each tile
         }
+        turns.init();
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -178,7 +225,10 @@ __global__ void __launch_bounds__(kThreads, NW >= 6 ? 1 : 2) k_stencils_tma(cons
             const int s0a = s0 & ~3, s1t = s1 & ~3;
             const int e0a = e0 & ~3, e1t = e1 & ~3;
             const bool staged = e1 >= e0 && (e1 - e0a) <= C::kCap;
-            if (lane == 0) meta[stage] = Meta{s0, s1, s0a, e0a, e1, staged ? 1 : 0};
+            if (lane == 0) {
+                turns.number(stage, it);
+                meta[stage] = Meta{s0, s1, s0a, e0a, e1, staged ? 1 : 0};
+            }
             uint32_t bytes = 0;
             if (s1t > s0a) bytes += (uint32_t)(s1t - s0a) * 8;
             if (staged && e1t > e0a) bytes += (uint32_t)(e1t - e0a) * 4 * (1 + NW);
@@ -224,8 +274,7 @@ __global__ void __launch_bounds__(kThreads, NW >= 6 ? 1 : 2) k_stencils_tma(cons
     int it = grp;
     for (int t = blockIdx.x + grp * gridDim.x; t < a.numTiles; t += G * gridDim.x, it += G) {
         const int stage = it % S;
-        const uint32_t use = (uint32_t)(it / S);
-        if (!mbar_wait(&full[stage], use & 1)) return;
+        if (!turns.wait(full, it)) return;
         int *sidx, *ssz, *sof;
         float *sw;
         stage_ptrs<NW>(smem, stage, &sidx, &sw, &ssz, &sof);
@@ -386,19 +435,21 @@ __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow
     extern __shared__ __align__(128) char smem[];
     using C = SellCfg<NW, VW>;
     constexpr int S = C::kRing, SPT = C::kSpt;
-    // consumer groups (one warp per slice of a tile), no more than the ring has stages: a group
-    // waits for its stage's use `it / S` by parity, which tells it from the use before only
+    // consumer groups (one warp per slice of a tile), no more than the ring has stages: the use
+    // before the last one of a group's stage is then complete (Turns)
     constexpr int G = 8 / SPT < S ? 8 / SPT : S;
     constexpr int GW = SPT;  // warps per group
     static_assert(G >= 1 && G <= S && G * GW <= kConsumers / 32, "consumer groups");
     __shared__ __align__(8) uint64_t full[S], empty[S];
     __shared__ SellMeta meta[S];
+    __shared__ Turns<S, G> turns;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int st = 0; st < S; ++st) {
             mbar_init(&full[st], 32);
             mbar_init(&empty[st], GW);
         }
+        turns.init();
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -425,6 +476,7 @@ __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow
             const int nslots = slot1 - slot0;
             const bool staged = nslots <= C::kSlots;
             if (lane == 0) {
+                turns.number(st, it);
                 meta[st] = SellMeta{s0, s1, slot0, staged ? 1 : 0};
                 const uint32_t pb = (uint32_t)(s1 - s0) * 128;
                 const uint32_t eb = staged ? (uint32_t)nslots * 4 : 0;
@@ -458,8 +510,7 @@ __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow
     int it = grp;
     for (int t = blockIdx.x + grp * gridDim.x; t < a.numTiles; t += G * gridDim.x, it += G) {
         const int st = it % S;
-        const uint32_t use = (uint32_t)(it / S);
-        if (!mbar_wait(&full[st], use & 1)) return;
+        if (!turns.wait(full, it)) return;
         int *ssz, *sor, *sidx;
         float *sw;
         stage(st, &ssz, &sor, &sidx, &sw);
