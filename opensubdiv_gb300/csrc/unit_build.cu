@@ -9,7 +9,6 @@
 //   4. slices: their size, the uniform ones verified bit for bit (a hash collision only costs
 //      the sharing), a scan of the blob sizes, then one warp per slice writes its blob.
 #include <climits>
-#include <vector>
 
 #include <cub/cub.cuh>
 
@@ -290,21 +289,28 @@ __global__ void __launch_bounds__(256) k_unit_fill(const Slices a, const int4 *m
     }
 }
 
-// Stream-ordered temporaries, released when the build returns.
+// Stream-ordered temporaries, released when the build returns, and the first failure: what comes
+// behind one works on nothing, so the steps that write by what an earlier one computed are not
+// queued any more.
 struct Temps {
     cudaStream_t s;
     const char *who;
-    std::vector<void *> p;
-    bool failed = false;
+    void *p[32] = {};
+    int status = GB300_OK;
+    bool failed() const { return status != GB300_OK; }
+    bool check(cudaError_t e) {
+        if (!failed()) status = check_cuda(e, who);
+        return !failed();
+    }
     template <class T>
     T *get(size_t count) {
-        void *q = nullptr;
-        if (scratch_alloc(&q, std::max<size_t>(count * sizeof(T), 16), s, who) != GB300_OK) {
-            failed = true;
-            return nullptr;
-        }
-        p.push_back(q);
-        return (T *)q;
+        void **slot = p;
+        while (slot < p + 32 && *slot) ++slot;
+        if (!failed() && slot == p + 32) status = fail(GB300_ERR_CUDA, "%s: temporaries", who);
+        if (failed()) return nullptr;
+        status = scratch_alloc(slot, std::max<size_t>(count * sizeof(T), 16), s, who);
+        if (failed()) *slot = nullptr;
+        return (T *)*slot;
     }
     void drop(void *q) {
         for (void *&x : p)
@@ -325,32 +331,37 @@ int build_units(int n, const int *sizes, const int *offsets, const int *indices,
     if (n <= 0 || n == INT_MAX) return n <= 0 ? ok() : GB300_ERR_UNSUPPORTED;
     typedef unsigned long long u64;
     const Csr c{sizes, offsets, indices, weights};
-    Temps tmp{s, who, {}, false};
+    Temps tmp{s, who};
+    auto launched = [&] {
+        count_launch();
+        tmp.check(cudaGetLastError());
+    };
     auto read = [&](auto *host, const auto *dev) {
-        if (check_cuda(cudaMemcpyAsync(host, dev, sizeof(*host), cudaMemcpyDeviceToHost, s), who) !=
-            GB300_OK)
-            return GB300_ERR_CUDA;
-        return check_cuda(cudaStreamSynchronize(s), who) == GB300_OK ? GB300_OK : GB300_ERR_CUDA;
+        if (!tmp.failed() &&
+            tmp.check(cudaMemcpyAsync(host, dev, sizeof(*host), cudaMemcpyDeviceToHost, s)))
+            tmp.check(cudaStreamSynchronize(s));
+        return tmp.status;
     };
     auto sort = [&](auto *kin, auto *kout, int *vin, int *vout, int count, int bits) {
         size_t bytes = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, bytes, kin, kout, vin, vout, count, 0, bits, s);
+        if (tmp.failed() || !tmp.check(cub::DeviceRadixSort::SortPairs(
+                                nullptr, bytes, kin, kout, vin, vout, count, 0, bits, s)))
+            return;
         void *q = tmp.get<char>(bytes);
         if (!q) return;
-        if (check_cuda(cub::DeviceRadixSort::SortPairs(q, bytes, kin, kout, vin, vout, count, 0,
-                                                       bits, s),
-                       who) != GB300_OK)
-            tmp.failed = true;
+        tmp.check(cub::DeviceRadixSort::SortPairs(q, bytes, kin, kout, vin, vout, count, 0, bits,
+                                                  s));
         count_launch();
         tmp.drop(q);
     };
     auto scan = [&](auto *in, auto *out, int count) {  // exclusive sum
         size_t bytes = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, count, s);
+        if (tmp.failed() ||
+            !tmp.check(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, count, s)))
+            return;
         void *q = tmp.get<char>(bytes);
         if (!q) return;
-        if (check_cuda(cub::DeviceScan::ExclusiveSum(q, bytes, in, out, count, s), who) != GB300_OK)
-            tmp.failed = true;
+        tmp.check(cub::DeviceScan::ExclusiveSum(q, bytes, in, out, count, s));
         count_launch();
         tmp.drop(q);
     };
@@ -362,31 +373,32 @@ int build_units(int n, const int *sizes, const int *offsets, const int *indices,
     // stencils in locality order, equal lists together
     u64 *hashW = tmp.get<u64>(n), *key = tmp.get<u64>(n), *key2 = tmp.get<u64>(n);
     int *iota = tmp.get<int>(n), *order = tmp.get<int>(n);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     k_unit_keys<<<grid_of(n, 256), 256, 0, s>>>(c, n, key, hashW, iota);
-    count_launch();
+    launched();
     sort(key, key2, iota, order, n, 64);
     int *flag = tmp.get<int>((size_t)n + 1), *group = tmp.get<int>((size_t)n + 1);
     int *groupAt = tmp.get<int>((size_t)n + 1);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     k_unit_heads<<<grid_of(n + 1LL, 256), 256, 0, s>>>(c, n, key2, order, flag);
-    count_launch();
+    launched();
     scan(flag, group, n + 1);
+    if (tmp.failed()) return tmp.status;
     k_unit_firsts<<<grid_of(n, 256), 256, 0, s>>>(group, n, groupAt);
-    count_launch();
+    launched();
     tmp.drop(key);
     tmp.drop(key2);
     tmp.drop(iota);
     // units
     int *id = tmp.get<int>((size_t)n + 1);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     k_unit_flags<<<grid_of(n + 1LL, 256), 256, 0, s>>>(c, n, most, order, group, groupAt, flag);
-    count_launch();
+    launched();
     scan(flag, id, n + 1);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     int *pos = groupAt;  // the groups are done with
     k_unit_firsts<<<grid_of(n, 256), 256, 0, s>>>(id, n, pos);
-    count_launch();
+    launched();
     int nu = 0;
     int st = read(&nu, id + n);
     if (st != GB300_OK) return st;
@@ -397,53 +409,53 @@ int build_units(int n, const int *sizes, const int *offsets, const int *indices,
     u64 *ukey = tmp.get<u64>(nu), *ukey2 = tmp.get<u64>(nu);
     int *uiota = tmp.get<int>(nu), *unit = tmp.get<int>(nu);
     unsigned *seg = tmp.get<unsigned>(nu), *seg2 = tmp.get<unsigned>(nu);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     k_unit_units<<<grid_of(nu, 256), 256, 0, s>>>(c, n, windowBits, order, id, pos, hashW, count,
                                                   ukey, uiota);
-    count_launch();
+    launched();
     sort(ukey, ukey2, uiota, unit, nu, 64);
+    if (tmp.failed()) return tmp.status;
     k_unit_segments<<<grid_of(nu, 256), 256, 0, s>>>(ukey2, unit, nu, windowBits, seg);
-    count_launch();
+    launched();
     sort(seg, seg2, unit, uiota, nu, windowBits + 2 + kPartBits);  // stable: key order kept
     unit = uiota;
     // slices
     int *sflag = tmp.get<int>((size_t)nu + 1), *sid = tmp.get<int>((size_t)nu + 1);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     k_unit_slices<<<grid_of(nu + 1LL, 256), 256, 0, s>>>(seg2, nu, sflag);
-    count_launch();
+    launched();
     scan(sflag, sid, nu + 1);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     int ns = 0;
     if ((st = read(&ns, sid + nu)) != GB300_OK) return st;
     int *firstOf = tmp.get<int>((size_t)ns + 1);
     long long *bytes = tmp.get<long long>((size_t)ns + 1), *start = tmp.get<long long>((size_t)ns + 1);
     int4 *meta = tmp.get<int4>(ns);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     k_unit_firsts<<<grid_of(nu, 256), 256, 0, s>>>(sid, nu, firstOf);
-    count_launch();
+    launched();
     unsigned *skey = tmp.get<unsigned>(ns), *skey2 = tmp.get<unsigned>(ns);
     int *siota = tmp.get<int>(ns), *at = tmp.get<int>(ns);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     k_unit_places<<<grid_of((long long)ns * 32, 256), 256, 0, s>>>(firstOf, unit, seg2, ns, nu, skey,
                                                                      siota);
-    count_launch();
+    launched();
     sort(skey, skey2, siota, at, ns, 32);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     u64 *shared = tmp.get<u64>(1);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     Slices a{c,     ns,    at,      firstOf, seg2,    unit, pos, count,
              order, start, bytes, shared,  nullptr, nullptr};
-    if (check_cuda(cudaMemsetAsync(bytes + ns, 0, 8, s), who) != GB300_OK ||
-        check_cuda(cudaMemsetAsync(shared, 0, 8, s), who) != GB300_OK)
-        return GB300_ERR_CUDA;
+    if (!tmp.check(cudaMemsetAsync(bytes + ns, 0, 8, s)) ||
+        !tmp.check(cudaMemsetAsync(shared, 0, 8, s)))
+        return tmp.status;
     k_unit_sizes<<<grid_of((long long)ns * 32, 256), 256, 0, s>>>(a, meta);
-    count_launch();
+    launched();
     scan(bytes, start, ns + 1);
-    if (tmp.failed) return GB300_ERR_OUT_OF_MEMORY;
+    if (tmp.failed()) return tmp.status;
     long long total = 0;
     u64 sharing = 0;
-    if ((st = check_launch(who)) != GB300_OK || (st = read(&total, start + ns)) != GB300_OK ||
-        (st = read(&sharing, shared)) != GB300_OK)
+    if ((st = read(&total, start + ns)) != GB300_OK || (st = read(&sharing, shared)) != GB300_OK)
         return st;
     if (total > INT_MAX) return GB300_ERR_UNSUPPORTED;
     auto fail_all = [&](int code) {
@@ -451,17 +463,16 @@ int build_units(int n, const int *sizes, const int *offsets, const int *indices,
             if (owned[k]) cudaFree(owned[k]), owned[k] = nullptr;
         return code;
     };
-    if (check_cuda(cudaMalloc(&owned[0], (size_t)ns * sizeof(int4)), who) != GB300_OK ||
-        check_cuda(cudaMalloc(&owned[1], (size_t)total * 128), who) != GB300_OK) {
+    if (!tmp.check(cudaMalloc(&owned[0], (size_t)ns * sizeof(int4))) ||
+        !tmp.check(cudaMalloc(&owned[1], (size_t)total * 128))) {
         cudaGetLastError();
-        return fail_all(GB300_ERR_OUT_OF_MEMORY);
+        return fail_all(tmp.status);
     }
     a.slice = (int4 *)owned[0];
     a.blob = (char *)owned[1];
     k_unit_fill<<<grid_of((long long)ns * 32, 256), 256, 0, s>>>(a, meta);
-    count_launch();
-    if (check_launch(who) != GB300_OK || check_cuda(cudaStreamSynchronize(s), who) != GB300_OK)
-        return fail_all(GB300_ERR_CUDA);
+    launched();
+    if (tmp.failed() || !tmp.check(cudaStreamSynchronize(s))) return fail_all(tmp.status);
     t.numSlices = ns;
     t.regular = sharing >= (u64)n / 2;
     t.numStencils = n;
