@@ -327,10 +327,19 @@ __global__ void __launch_bounds__(kThreads, (Ring<CLS, SLICED>::kMinBlocks))
     if (warp == kConsumers / 32) {
         // producer: claim tiles until the list is exhausted, then post one "done" stage
         int jc = 0;  // job of the last claimed tile (claims only grow)
+        // Before the producer leaves: the copies still on their way into the shared memory, which
+        // is another CTA's afterwards, should the consumers have left at an expired wait.
+        auto drain = [&](int stages) {  // that have been filled
+            for (int k = max(stages - S, 0); k < stages; ++k)
+                bar_wait(&full[k % S], (uint32_t)(k / S) & 1, a.status);
+        };
         for (int it = 0;; ++it) {
             const int stage = it % S;
             const uint32_t use = (uint32_t)(it / S);
-            if (use > 0 && !bar_wait(&empty[stage], (use - 1) & 1, a.status)) return;
+            if (use > 0 && !bar_wait(&empty[stage], (use - 1) & 1, a.status)) {
+                drain(it);
+                return;
+            }
             int t = (int)blockIdx.x + it * (int)gridDim.x;
             if (a.dynamic) {
                 if (lane == 0) t = atomicAdd(a.counter, 1);
@@ -343,6 +352,7 @@ __global__ void __launch_bounds__(kThreads, (Ring<CLS, SLICED>::kMinBlocks))
                 if (lane == 0) meta[stage] = Meta{0, 0, 0, 0, 0, 0, 0, 1};
                 __syncwarp();
                 bar_arrive(&full[stage]);  // all 32 lanes: completes the phase without tx
+                drain(it + 1);             // this stage's phase is the end's
                 return;
             }
             // advance jc to the last job whose first tile is <= t (tileBase is non-decreasing,
@@ -511,7 +521,10 @@ __global__ void __launch_bounds__(units::kThreads, 1) k_stencils_batch_units(con
         }
         if (f.popped == f.pushed) return;
         const int s = f.popped % kAhead;
-        if (!ring::wait(&q.full[s], (uint32_t)(f.popped / kAhead) & 1, a.status)) return;
+        if (!ring::wait(&q.full[s], (uint32_t)(f.popped / kAhead) & 1, a.status)) {
+            drain(q, f, far, a.status);
+            return;
+        }
         const Job &j = a.jobs[slotJob[warp][s]];
         struct View {
             const float *src;
@@ -520,8 +533,10 @@ __global__ void __launch_bounds__(units::kThreads, 1) k_stencils_batch_units(con
         };
         const View v{j.src, {j.dst[0]}, {j.dstStride[0]}, j.srcStride, j.length};
         if (!consume<COLLECT>(v, q, bytes, reinterpret_cast<const char *>(j.slIdx), far, s, lane,
-                     unit_shift(v.length), pol_stream, a.status))
+                              unit_shift(v.length), pol_stream, a.status)) {
+            drain(q, f, far, a.status);
             return;
+        }
         __syncwarp();
     }
 }

@@ -78,6 +78,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity) {
     }
     return true;
 }
+// Before a producer that has filled `tiles` stages leaves: the copies still on their way into the
+// shared memory, which is another CTA's afterwards, should the consumers have left at an expired
+// wait.  Each wait has the same limit again.
+template <int S>
+__device__ __forceinline__ void drain(uint64_t *full, int tiles) {
+    for (int k = max(tiles - S, 0); k < tiles; ++k)
+        mbar_wait(full + k % S, (uint32_t)(k / S) & 1);
+}
 // A consumer group's wait for its tile `it` in a ring of S stages that G groups take turns on.  The
 // use of the stage is told by its parity, which tells it from the use before only if that one has
 // completed.  With S a multiple of G the group consumed that one itself.  Else it was another
@@ -209,7 +217,7 @@ __global__ void __launch_bounds__(kThreads, NW >= 6 ? 1 : 2) k_stencils_tma(cons
         for (int t = blockIdx.x; t < a.numTiles; t += gridDim.x, ++it) {
             const int stage = it % S;
             const uint32_t use = (uint32_t)(it / S);
-            if (use > 0 && !mbar_wait(&empty[stage], (use - 1) & 1)) return;
+            if (use > 0 && !mbar_wait(&empty[stage], (use - 1) & 1)) break;
             int *sidx, *ssz, *sof;
             float *sw;
             stage_ptrs<NW>(smem, stage, &sidx, &sw, &ssz, &sof);
@@ -264,6 +272,7 @@ __global__ void __launch_bounds__(kThreads, NW >= 6 ? 1 : 2) k_stencils_tma(cons
             __syncwarp();
             if (lane != 0) mbar_arrive(&full[stage]);
         }
+        drain<S>(full, it);
         return;
     }
 
@@ -467,7 +476,7 @@ __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow
         for (int t = blockIdx.x; t < a.numTiles; t += gridDim.x, ++it) {
             const int st = it % S;
             const uint32_t use = (uint32_t)(it / S);
-            if (use > 0 && !mbar_wait(&empty[st], (use - 1) & 1)) return;
+            if (use > 0 && !mbar_wait(&empty[st], (use - 1) & 1)) break;
             int *ssz, *sor, *sidx;
             float *sw;
             stage(st, &ssz, &sor, &sidx, &sw);
@@ -494,6 +503,7 @@ __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow
             __syncwarp();
             if (lane != 0) mbar_arrive(&full[st]);
         }
+        drain<S>(full, it);
         return;
     }
     // consumers: group g takes this CTA's tiles it = g, g + G, ...; warp wg of the group takes

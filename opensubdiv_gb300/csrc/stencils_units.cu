@@ -60,9 +60,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_stencils_units(const Args arg) 
         wait = false;
         if (f.popped == f.pushed) return;
         const int s = f.popped % kAhead;
-        if (!ring::wait(&q.full[s], (uint32_t)(f.popped / kAhead) & 1, a.status)) return;
-        if (!consume<COLLECT>(a, q, bytes, a.blob, far, s, lane, a.shift, pol_stream, a.status))
+        if (!ring::wait(&q.full[s], (uint32_t)(f.popped / kAhead) & 1, a.status) ||
+            !consume<COLLECT>(a, q, bytes, a.blob, far, s, lane, a.shift, pol_stream, a.status)) {
+            drain(q, f, far, a.status);
             return;
+        }
         __syncwarp();
     }
 }

@@ -123,6 +123,15 @@ __device__ __forceinline__ bool consume(const A &a, const Queue &q, const char *
     }
 }
 
+// Behind an expired wait: the copies that are still on their way into this warp's shared memory,
+// which is another CTA's when this one has left, each waited for with a limit again.
+__device__ __forceinline__ void drain(Queue &q, const Feed &f, const Far &far, int *status) {
+    for (int k = f.popped; k < f.pushed; ++k)
+        ring::wait(&q.full[k % kAhead], (uint32_t)(k / kAhead) & 1, status);
+    for (int k = far.used; k < far.issued; ++k)
+        ring::wait(&q.far[k % kFarBlocks], (uint32_t)(k / kFarBlocks) & 1, status);
+}
+
 // Lanes that share a unit of a primvar `length` floats wide: one per 4 columns, 4 at most.
 __host__ __device__ inline int unit_shift(int length) { return length <= 4 ? 0 : length <= 8 ? 1 : 2; }
 
