@@ -6,7 +6,10 @@
 // (descending, stable) within windows of 256 positions so that the 32 stencils of a slice have
 // similar sizes.  Slice s covers positions [32 s, 32 s + 32); its width is the largest size of
 // its stencils, and entry j of the stencil at lane l sits in slot sliceSlot[s] + 32 j + l
-// (slots past a stencil's size hold index 0 / weight 0 and are never read).
+// Slots past a stencil's size hold weight 0.  Those of an empty stencil (or of none) hold an index
+// that its slice reads anyway: kernels of several outputs load the row of a lane's last entry in
+// steps past it, of its first slot where it has none, and a row that the table does not name may
+// lie outside the caller's buffer.  The other slots past a size hold 0 and are not read.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -21,6 +24,13 @@ struct SellTable {
     const float *w[6] = {};          // slots, per weight array of the table
     const int *outRow = nullptr;     // numSlices * 32: destination stencil (-1: padding)
 };
+
+// The index in the slots of an empty stencil of slice `s`: the slice's first, whose stencil is its
+// longest.
+__host__ __device__ inline int sell_pad_index(const int *indices, const int *offsets, const int *row,
+                                              long long s, int width) {
+    return width > 0 ? indices[offsets[row[s * 32]]] : 0;
+}
 
 // Builds the layout of the device CSR table (sizes, offsets, indices, up to 6 weight arrays,
 // entries sorted per stencil for the locality order to mean anything) on stream `s` and waits

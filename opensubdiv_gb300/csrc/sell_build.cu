@@ -85,8 +85,8 @@ struct Weights {
     float *out[6];
 };
 
-// Thread per position: its stencil's entries into slots start[s] + 32 j + lane (zeros past the
-// stencil's size up to the slice width); lane 0 of each slice records the 32-bit slot offset.
+// Thread per position: its stencil's entries into slots start[s] + 32 j + lane (past the stencil's
+// size up to the slice width: weight 0, and an index as sell.h says); lane 0 of each slice records the 32-bit slot offset.
 __global__ void k_fill(const int *sz, const int *row, const long long *start, int ns,
                        const int *offsets, const int *indices, Weights w, int *sliceSlot,
                        int *idx) {
@@ -100,10 +100,11 @@ __global__ void k_fill(const int *sz, const int *row, const long long *start, in
         if (p == 0) sliceSlot[ns] = (int)start[ns];
         const int n = sz[p], r = row[p];
         const long long o = r >= 0 ? offsets[r] : 0;
+        const int pad = n > 0 ? 0 : sell_pad_index(indices, offsets, row, sl, width);
         for (int j = 0; j < width; ++j) {
             const long long slot = b + 32LL * j + lane;
             const bool on = j < n;
-            idx[slot] = on ? indices[o + j] : 0;
+            idx[slot] = on ? indices[o + j] : pad;
 #pragma unroll
             for (int k = 0; k < 6; ++k)
                 if (w.in[k]) w.out[k][slot] = on ? w.in[k][o + j] : 0.0f;
