@@ -134,25 +134,33 @@ __device__ __forceinline__ float ld_stream(const float *p, uint64_t pol) {
 }
 
 // Coherent loads of the caller's data, which a kernel queued before may write.  Two forms keep them
-// behind wait_for_primary: the volatile ones stand where the program has them, among themselves and
-// against the wait; the others the compiler may move, as far as their address allows, which is to
-// come from behind_wait.  (EvalPatches, 4 M points: lanes with volatile rows and indices 374 -> 396
-// us, their loads no longer overlapping as the compiler had them; Loop rows through behind_wait 255
-// -> 261 us, for the registers of the pointer.)
+// behind wait_for_primary: the volatile ones keep their order among themselves and with the wait;
+// the others the compiler may move, as far as their address allows, which is to come from
+// behind_wait.  (EvalPatches, 4 M points: lanes with volatile rows and indices 374 -> 396 us, their
+// loads no longer overlapping as the compiler had them.  Elsewhere the pointer's registers cost more:
+// Loop rows through behind_wait 255 -> 261 us, three outputs of 4-wide stencil rows 18.7 -> 20.5.)
 //
 // Source rows: kept in L1, evict-last in L2 (the control points are re-read by every stencil that
 // touches them).
 __device__ __forceinline__ float ld_src(const float *p, uint64_t pol) {
     float v;
-    asm("ld.global.L1::evict_last.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L1::evict_last.L2::cache_hint.f32 %0, [%1], %2;"
+                 : "=f"(v)
+                 : "l"(p), "l"(pol));
     return v;
 }
 __device__ __forceinline__ float4 ld_src4(const float *p) {
     float4 v;
-    asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-        : "l"(p));
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p));
     return v;
+}
+__device__ __forceinline__ void ld_src8(const float *p, float (&x)[8]) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]),
+                   "=f"(x[6]), "=f"(x[7])
+                 : "l"(p));
 }
 __device__ __forceinline__ float4 ld_row4(const float *p, uint64_t pol) {
     float4 v;
@@ -162,7 +170,25 @@ __device__ __forceinline__ float4 ld_row4(const float *p, uint64_t pol) {
                  : "memory");
     return v;
 }
-// Indices of patches.
+// Movable: rows in a unit or a batched slice, elements and indices of patches.
+__device__ __forceinline__ void ld_point8(const float *p, float (&x)[8]) {
+    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]),
+          "=f"(x[7])
+        : "l"(p));
+}
+__device__ __forceinline__ float4 ld_point4(const float *p) {
+    float4 v;
+    asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_point(const float *p, uint64_t pol) {
+    float v;
+    asm("ld.global.L1::evict_last.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+    return v;
+}
 __device__ __forceinline__ int ld_keep(const int *p, uint64_t pol) {
     int v;
     asm("ld.global.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));

@@ -77,7 +77,7 @@ __device__ __forceinline__ void load_row(const float *src, int stride, int cv,
         if constexpr (LC == 4) x[3] = v.w;
     } else {
 #pragma unroll
-        for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? ld_src(p + c, pol) : 0.0f;
+        for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? ld_point(p + c, pol) : 0.0f;
     }
 }
 
@@ -100,7 +100,7 @@ __device__ __forceinline__ void load_row(const float *src, int stride, int cv,
         const float *p = src + (size_t)cv * stride + e0;
         const uint64_t pol = l2_evict_last();
 #pragma unroll
-        for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? ld_src(p + c, pol) - xc[c] : 0.0f;
+        for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? ld_point(p + c, pol) - xc[c] : 0.0f;
     }
 }
 

@@ -8,39 +8,40 @@
 namespace gb300 {
 namespace tma {
 
-// Source rows are read with coherent loads: kernels queued before may write them (launch_kernel).
-//
 // Elements [c0, c0 + 8) of source row `id` (zeros past the primvar length): one 256-bit load
 // for 32-byte aligned rows, two 128-bit loads for 16-byte aligned rows, else scalar loads.
-// VW = 0 picks the width at run time from a.vw (one code path for jobs of mixed layouts).
-template <int VW, class A>
+// VW = 0 picks the width at run time from a.vw (one code path for jobs of mixed layouts).  Coherent
+// loads, kernels queued before may write the rows (launch_kernel); MOVABLE ones in the batched
+// kernels, which are launched behind all earlier work.
+template <int VW, class A, bool MOVABLE = false>
 __device__ __forceinline__ void gather_row(const A &a, int id, int c0, uint64_t pol_src,
                                            float (&x)[8]) {
     const float *row = a.src + (size_t)id * a.srcStride + c0;
     if constexpr (VW == 0) {
         if (a.vw == 8)
-            gather_row<8>(a, id, c0, pol_src, x);
+            gather_row<8, A, true>(a, id, c0, pol_src, x);
         else if (a.vw == 4)
-            gather_row<4>(a, id, c0, pol_src, x);
+            gather_row<4, A, true>(a, id, c0, pol_src, x);
         else
-            gather_row<1>(a, id, c0, pol_src, x);
+            gather_row<1, A, true>(a, id, c0, pol_src, x);
     } else if constexpr (VW == 8) {
-        asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                     : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]),
-                       "=f"(x[6]), "=f"(x[7])
-                     : "l"(row));
+        if constexpr (MOVABLE) ld_point8(row, x);
+        else ld_src8(row, x);
     } else if constexpr (VW == 4) {
-        const float4 v0 = ld_src4(row);
+        const float4 v0 = MOVABLE ? ld_point4(row) : ld_src4(row);
         x[0] = v0.x; x[1] = v0.y; x[2] = v0.z; x[3] = v0.w;
         if (c0 + 4 < a.length) {
-            const float4 v1 = ld_src4(row + 4);
+            const float4 v1 = MOVABLE ? ld_point4(row + 4) : ld_src4(row + 4);
             x[4] = v1.x; x[5] = v1.y; x[6] = v1.z; x[7] = v1.w;
         } else {
             x[4] = x[5] = x[6] = x[7] = 0.0f;
         }
     } else {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) x[c] = (c0 + c < a.length) ? ld_src(row + c, pol_src) : 0.0f;
+        for (int c = 0; c < 8; ++c)
+            x[c] = c0 + c >= a.length ? 0.0f
+                   : MOVABLE          ? ld_point(row + c, pol_src)
+                                      : ld_src(row + c, pol_src);
     }
 }
 

@@ -368,11 +368,6 @@ struct SellArgs {
     unsigned magic;  // 65536 / length + 1
 };
 
-struct SourceRows {  // gather_row's view
-    const float *src;
-    int srcStride, length;
-};
-
 struct SellMeta {
     int s0, s1, slot0, staged;
 };
@@ -381,7 +376,7 @@ struct SellMeta {
 // 16-byte loads; the row stride is a multiple of 4 floats, at least 12), or the 4 columns of a
 // row of at most 4 floats (VW = kNarrow: one 16-byte load, stride a multiple of 4).
 template <int VW>
-__device__ __forceinline__ void gather_cols(const SourceRows &a, int id, int c0, uint64_t pol_src,
+__device__ __forceinline__ void gather_cols(const SellArgs &a, int id, int c0, uint64_t pol_src,
                                             float (&x)[VW == 12 ? 12 : VW == kNarrow ? 4 : 8]) {
     if constexpr (VW == kNarrow) {
         const float4 q = ld_src4(a.src + (size_t)id * a.srcStride + c0);
@@ -512,8 +507,6 @@ __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow
     if (grp >= G) return;
     // the producer streams the table, which no queued work writes, while the kernel before ends
     wait_for_primary();
-    SourceRows rows{a.src, a.srcStride, a.length};
-    behind_wait(rows.src);
     // entry steps gathered together, columns per pass
     constexpr int R = VW == kNarrow ? (NW == 1 ? 6 : 4) : VW == 12 ? 2 : NW <= 3 ? 4 : 2;
     constexpr int CW = VW == 12 ? 12 : VW == kNarrow ? 4 : 8;
@@ -567,7 +560,7 @@ __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow
                     float x[R][CW];
 #pragma unroll
                     for (int q = 0; q < R; ++q)
-                        if (!SKIP || j0 + q < n) gather_cols<VW>(rows, ids[q], c0, pol_src, x[q]);
+                        if (!SKIP || j0 + q < n) gather_cols<VW>(a, ids[q], c0, pol_src, x[q]);
 #pragma unroll
                     for (int q = 0; q < R; ++q)
                         if (j0 + q < n)

@@ -22,7 +22,7 @@ namespace units {
 // floats (columns at or past the length, inside the stride, are read and not used).
 template <class A>
 __device__ __forceinline__ float4 load_quad(const A &a, int id, int c0) {
-    return ld_src4(a.src + (size_t)id * a.srcStride + c0);
+    return ld_point4(a.src + (size_t)id * a.srcStride + c0);
 }
 
 // Output rows are 16-byte aligned, their stride a multiple of 4 floats.

@@ -79,24 +79,31 @@ def test_non_coherent_instructions_are_in_the_named_loads_only():
 
 
 def test_coherent_loads_stay_behind_the_wait():
-    """An asm load is volatile with a memory clobber, or one of those whose addresses the dependent
-    kernels take from behind_wait: a source pointer in each of them, the patch indices."""
-    movable = set()
+    """An asm load is volatile, as the wait is, or one of those whose addresses the dependent kernels
+    take from behind_wait: rows of units, EvalPatches' source elements and patch indices."""
+    movable = {}
     for path in glob.glob(CSRC + "/*.cu*"):
         text = _code(path)
         for m in re.finditer(r"asm\s*(volatile)?\s*\((.*?)\);", text, flags=re.S):
             if "ld.global" in m.group(2) and ".nc" not in m.group(2) and m.group(1) is None:
-                movable.add(re.findall(r"__device__[^\n]*?(\w+)\(", text[:m.start()])[-1])
-            elif "ld.global" in m.group(2) and ".nc" not in m.group(2):
-                assert '"memory"' in m.group(2), m.group(2)
-    assert movable == {"ld_src", "ld_src4", "ld_keep", "ld_keep4", "gather_row"}
-    for name, pointers in (("stencils_tma.cu", ["rows.src"]), ("stencils_units.cu", ["a.src"]),
-                           ("patches.cu", ["a.src", "a.indices"])):
-        text = _code(os.path.join(CSRC, name))
-        for p in pointers:
-            assert f"behind_wait({p})" in text, (name, p)
+                load = re.findall(r"__device__[^\n]*?(\w+)\(", text[:m.start()])[-1]
+                movable[load] = os.path.basename(path)
+    assert movable == dict.fromkeys(("ld_point", "ld_point4", "ld_point8", "ld_keep", "ld_keep4"), "common.cuh")
+    for path in glob.glob(CSRC + "/*.cu*"):
+        if re.search(r"\b(ld_point[48]?|ld_keep4?)\(", _code(path)):
+            assert os.path.basename(path) in ("common.cuh", "patch_basis.cuh", "unit_eval.cuh",
+                                              "stencil_eval.cuh"), path
+    # stencil_eval.cuh's are for the batched kernels, which are not dependents
+    for name in ("stencils_tma.cu", "stencils_units.cu"):
+        assert not re.search(r"gather_row<0>|true>\(a, id", _code(os.path.join(CSRC, name)))
+    assert "launch_kernel(k_stencils_batch" not in _code(os.path.join(CSRC, "stencils_batch.cu"))
+    assert "behind_wait(a.src)" in _code(os.path.join(CSRC, "stencils_units.cu"))
     text = _code(os.path.join(CSRC, "patches.cu"))
+    assert "behind_wait(a.src)" in text and "behind_wait(a.indices)" in text
     assert text.count("= args_behind_wait<") == len(re.findall(r"\bk_eval_patches\w*\(const", text))
+    # the wait itself is volatile too
+    common = _code(os.path.join(CSRC, "common.cuh"))
+    assert 'asm volatile("griddepcontrol.wait;" ::: "memory")' in common
 
 
 def test_row_pointers_are_not_restrict():
