@@ -92,7 +92,8 @@ int once_per_device(std::atomic<uint64_t> &done, F fn) {
 
 // Programmatic dependent launch (launch_kernel).  launch_dependents lets the next kernel be started
 // as soon as every CTA of this one runs; it is then resident, and waits in wait_for_primary until
-// this one is done and its writes are visible.
+// this one is done and its writes are visible.  A kernel that calls it before it waits itself lets
+// the chain behind it start as well.
 __device__ __forceinline__ void launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
