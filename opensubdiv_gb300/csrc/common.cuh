@@ -171,7 +171,7 @@ __device__ __forceinline__ float4 ld_row4(const float *p, uint64_t pol) {
                  : "memory");
     return v;
 }
-// Movable: rows in a unit or a batched slice, elements and indices of patches.
+// Movable: rows in a unit or a batched slice, elements and indices of patches read by lanes.
 __device__ __forceinline__ void ld_point8(const float *p, float (&x)[8]) {
     asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]),
@@ -190,16 +190,26 @@ __device__ __forceinline__ float ld_point(const float *p, uint64_t pol) {
     asm("ld.global.L1::evict_last.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
     return v;
 }
-__device__ __forceinline__ int ld_keep(const int *p, uint64_t pol) {
+template <bool MOVABLE>
+__device__ __forceinline__ int ld_index(const int *p, uint64_t pol) {
     int v;
-    asm("ld.global.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+    if constexpr (MOVABLE)
+        asm("ld.global.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+    else
+        asm volatile("ld.global.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
     return v;
 }
-__device__ __forceinline__ int4 ld_keep4(const int *p, uint64_t pol) {
+template <bool MOVABLE>
+__device__ __forceinline__ int4 ld_index4(const int *p, uint64_t pol) {
     int4 v;
-    asm("ld.global.L2::cache_hint.v4.b32 {%0, %1, %2, %3}, [%4], %5;"
-        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-        : "l"(p), "l"(pol));
+    if constexpr (MOVABLE)
+        asm("ld.global.L2::cache_hint.v4.b32 {%0, %1, %2, %3}, [%4], %5;"
+            : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+            : "l"(p), "l"(pol));
+    else
+        asm volatile("ld.global.L2::cache_hint.v4.b32 {%0, %1, %2, %3}, [%4], %5;"
+                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "l"(p), "l"(pol));
     return v;
 }
 // Params of patches, and queries (read once: no L1 allocation).

@@ -56,9 +56,17 @@ struct Acc6 {
 // points, from src on, so that no index is read.
 enum SourceRows { kAnyRows = 0, kQuadRows = 1, kPatchRows = 2 };
 
-template <int V4>
+template <int LC, int V4>
 __device__ __forceinline__ int row_index(const int *cvs, int j) {
-    return V4 == kPatchRows ? j : ld_keep(cvs + j, l2_evict_last());
+    return V4 == kPatchRows ? j : ld_index<LC == 1>(cvs + j, l2_evict_last());
+}
+
+// One element: movable where a row is one (the lanes' loads overlap as the compiler has them),
+// volatile where rows are wider (the pointer's registers cost more; P and the first derivatives of
+// 2 M Loop points 142 and 138 us).
+template <int LC>
+__device__ __forceinline__ float load_element(const float *p, uint64_t pol) {
+    return LC == 1 ? ld_point(p, pol) : ld_src(p, pol);
 }
 
 // Loads LC elements [e0, e0+LC) of control point `cv` (elements >= length read as 0): quads in one
@@ -77,7 +85,7 @@ __device__ __forceinline__ void load_row(const float *src, int stride, int cv,
         if constexpr (LC == 4) x[3] = v.w;
     } else {
 #pragma unroll
-        for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? ld_point(p + c, pol) : 0.0f;
+        for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? load_element<LC>(p + c, pol) : 0.0f;
     }
 }
 
@@ -100,7 +108,7 @@ __device__ __forceinline__ void load_row(const float *src, int stride, int cv,
         const float *p = src + (size_t)cv * stride + e0;
         const uint64_t pol = l2_evict_last();
 #pragma unroll
-        for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? ld_point(p + c, pol) - xc[c] : 0.0f;
+        for (int c = 0; c < LC; ++c) x[c] = (e0 + c < length) ? load_element<LC>(p + c, pol) - xc[c] : 0.0f;
     }
 }
 
@@ -112,7 +120,7 @@ __device__ __forceinline__ void add_origin(const float (&xc)[LC], Acc6<LC> &acc)
 
 // N control-point indices of a patch: 128-bit loads when the index row is 16-byte aligned
 // (REGULAR rows are 64 B, GREGORY_BASIS rows 80 B), scalar loads otherwise.
-template <int N, int V4>
+template <int N, int LC, int V4>
 __device__ __forceinline__ void load_indices(const int *cvs, int (&idx)[N]) {
     if constexpr (V4 == kPatchRows) {
 #pragma unroll
@@ -123,12 +131,12 @@ __device__ __forceinline__ void load_indices(const int *cvs, int (&idx)[N]) {
     if ((N % 4) == 0 && (reinterpret_cast<uintptr_t>(cvs) & 15) == 0) {
 #pragma unroll
         for (int j = 0; j < N / 4; ++j) {
-            const int4 v = ld_keep4(cvs + 4 * j, pol);
+            const int4 v = ld_index4<LC == 1>(cvs + 4 * j, pol);
             idx[4 * j] = v.x; idx[4 * j + 1] = v.y; idx[4 * j + 2] = v.z; idx[4 * j + 3] = v.w;
         }
     } else {
 #pragma unroll
-        for (int j = 0; j < N; ++j) idx[j] = ld_keep(cvs + j, pol);
+        for (int j = 0; j < N; ++j) idx[j] = ld_index<LC == 1>(cvs + j, pol);
     }
 }
 
@@ -209,7 +217,7 @@ __device__ void eval_bspline(float s, float t, int boundary, const int *cvs,
     if (boundary & 4) { fold_last(tp); fold_last(td); fold_last(tdd); }
     if (boundary & 8) { fold_first(sp); fold_first(sd); fold_first(sdd); }
     int idx[16];
-    load_indices<16, V4>(cvs, idx);
+    load_indices<16, LC, V4>(cvs, idx);
     float xc[LC];  // point 5: the patch's (0,0) corner, never a phantom
     if constexpr (LC == 1) {  // all 16 rows in flight at a time
         float x[16][1];
@@ -254,7 +262,7 @@ __device__ void eval_gregory(float s, float t, const int *cvs,
     float d3 = s + tc;  d3 = (d3 <= 0.0f) ? 1.0f : (1.0f / d3);
     const float g0 = s * d0, g2 = t * d1, g4 = sc * d2, g6 = tc * d3;
     int idx[20];
-    load_indices<20, V4>(cvs, idx);
+    load_indices<20, LC, V4>(cvs, idx);
     float xc[LC];  // point 0: the patch's (0,0) corner
     load_row<LC, V4>(src, stride, idx[0], e0, length, xc);
     // rows of the Bezier grid; interior entries are blended pairs
@@ -350,20 +358,20 @@ __device__ void eval_gregory_tri(float s, float t, const int *cvs,
     // Bezier point m comes from Gregory point kBez[m] (or a blended pair for 6, 7, 10)
     constexpr int kBez[15] = {0, 1, 15, 7, 5, 2, -1, -2, 6, 17, -3, 16, 11, 12, 10};
     float xc[LC];  // point 0: the (0,0) corner
-    load_row<LC, V4>(src, stride, row_index<V4>(cvs, 0), e0, length, xc);
+    load_row<LC, V4>(src, stride, row_index<LC, V4>(cvs, 0), e0, length, xc);
     float B[15][LC];
 #pragma unroll
     for (int m = 0; m < 15; ++m) {
         const int gi = kBez[m];
         if (gi >= 0) {
-            load_row<LC, V4>(src, stride, row_index<V4>(cvs, gi), e0, length, B[m], xc);
+            load_row<LC, V4>(src, stride, row_index<LC, V4>(cvs, gi), e0, length, B[m], xc);
         } else {
             const int a = (gi == -1) ? 3 : (gi == -2) ? 8 : 13;
             const float ga = (gi == -1) ? g[0] : (gi == -2) ? g[2] : g[4];
             const float gb = (gi == -1) ? g[1] : (gi == -2) ? g[3] : g[5];
             float xa[LC], xb[LC];
-            load_row<LC, V4>(src, stride, row_index<V4>(cvs, a), e0, length, xa, xc);
-            load_row<LC, V4>(src, stride, row_index<V4>(cvs, a + 1), e0, length, xb, xc);
+            load_row<LC, V4>(src, stride, row_index<LC, V4>(cvs, a), e0, length, xa, xc);
+            load_row<LC, V4>(src, stride, row_index<LC, V4>(cvs, a + 1), e0, length, xb, xc);
 #pragma unroll
             for (int c = 0; c < LC; ++c) B[m][c] = ga * xa[c] + gb * xb[c];
         }
@@ -498,7 +506,7 @@ __device__ void eval_box_tri(float s, float t, int boundary, const int *cvs,
     float x[12][LC], xc[LC];
     {
         int idx[12];
-        load_indices<12, V4>(cvs, idx);
+        load_indices<12, LC, V4>(cvs, idx);
         load_row<LC, V4>(src, stride, idx[4], e0, length, xc);  // point 4: the (0,0) corner
 #pragma unroll
         for (int j = 0; j < 12; ++j) load_row<LC, V4>(src, stride, idx[j], e0, length, x[j], xc);
@@ -528,11 +536,11 @@ __device__ void eval_linear_quad(float s, float t, const int *cvs,
     const float wt[4] = {-sc, -s, s, sc};
     const float wst[4] = {1.0f, -1.0f, 1.0f, -1.0f};
     float xc[LC];
-    load_row<LC, V4>(src, stride, row_index<V4>(cvs, 0), e0, length, xc);
+    load_row<LC, V4>(src, stride, row_index<LC, V4>(cvs, 0), e0, length, xc);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         float x[LC];
-        load_row<LC, V4>(src, stride, row_index<V4>(cvs, j), e0, length, x, xc);
+        load_row<LC, V4>(src, stride, row_index<LC, V4>(cvs, j), e0, length, x, xc);
 #pragma unroll
         for (int c = 0; c < LC; ++c) {
             acc.v[0][c] = fmaf(wp[j], x[c], acc.v[0][c]);
@@ -549,9 +557,9 @@ __device__ void eval_linear_tri(float s, float t, const int *cvs,
                                 const float *src, int stride, int e0, int length,
                                 Acc6<LC> &acc) {
     float x0[LC], x1[LC], x2[LC];
-    load_row<LC, V4>(src, stride, row_index<V4>(cvs, 0), e0, length, x0);
-    load_row<LC, V4>(src, stride, row_index<V4>(cvs, 1), e0, length, x1, x0);
-    load_row<LC, V4>(src, stride, row_index<V4>(cvs, 2), e0, length, x2, x0);
+    load_row<LC, V4>(src, stride, row_index<LC, V4>(cvs, 0), e0, length, x0);
+    load_row<LC, V4>(src, stride, row_index<LC, V4>(cvs, 1), e0, length, x1, x0);
+    load_row<LC, V4>(src, stride, row_index<LC, V4>(cvs, 2), e0, length, x2, x0);
     // relative to point 0: P = x0 + s (x1 - x0) + t (x2 - x0)
 #pragma unroll
     for (int c = 0; c < LC; ++c) {

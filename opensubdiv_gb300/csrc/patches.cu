@@ -54,11 +54,13 @@ struct PatchArgs {
 };
 
 // The arguments with the pointers whose loads may move as they stand behind the wait.
-template <int V4>
+template <int LC, int V4>
 __device__ __forceinline__ PatchArgs args_behind_wait(const PatchArgs &arg) {
     PatchArgs a = arg;
-    if (V4 == kAnyRows) behind_wait(a.src);
-    if (V4 != kPatchRows) behind_wait(a.indices);
+    if (LC == 1) {
+        behind_wait(a.src);
+        behind_wait(a.indices);
+    }
     return a;
 }
 
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(128, LC == 4 ? 4 : (ORDER < 2 && !V4 ? (QUAD ?
     k_eval_patches(const PatchArgs arg) {
     launch_dependents();
     wait_for_primary();
-    const PatchArgs a = args_behind_wait<V4>(arg);
+    const PatchArgs a = args_behind_wait<LC, V4>(arg);
     constexpr bool PACK = LC > 1 && (!QUAD || V4);
     const int stride = gridDim.x * blockDim.x;
     if constexpr (!PACK) {
@@ -180,7 +182,7 @@ template <int G, int ORDER>
 __global__ void __launch_bounds__(256, 4) k_eval_patches_lanes(const PatchArgs arg) {
     launch_dependents();
     wait_for_primary();
-    const PatchArgs a = args_behind_wait<kAnyRows>(arg);
+    const PatchArgs a = args_behind_wait<1, kAnyRows>(arg);
     // G need not be a power of two: a warp holds floor(32 / G) groups (3 lanes per point
     // for xyz: 10 points per warp) and its remaining lanes stay idle
     constexpr int kPerWarp = 32 / G;

@@ -88,9 +88,10 @@ def test_coherent_loads_stay_behind_the_wait():
             if "ld.global" in m.group(2) and ".nc" not in m.group(2) and m.group(1) is None:
                 load = re.findall(r"__device__[^\n]*?(\w+)\(", text[:m.start()])[-1]
                 movable[load] = os.path.basename(path)
-    assert movable == dict.fromkeys(("ld_point", "ld_point4", "ld_point8", "ld_keep", "ld_keep4"), "common.cuh")
+    assert movable == dict.fromkeys(("ld_point", "ld_point4", "ld_point8", "ld_index",
+                                     "ld_index4"), "common.cuh")
     for path in glob.glob(CSRC + "/*.cu*"):
-        if re.search(r"\b(ld_point[48]?|ld_keep4?)\(", _code(path)):
+        if re.search(r"\b(ld_point[48]?|ld_index4?)\(", _code(path)):
             assert os.path.basename(path) in ("common.cuh", "patch_basis.cuh", "unit_eval.cuh",
                                               "stencil_eval.cuh"), path
     # stencil_eval.cuh's are for the batched kernels, which are not dependents
