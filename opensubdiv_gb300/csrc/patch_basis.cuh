@@ -204,7 +204,7 @@ __device__ __forceinline__ void tensor_accumulate(const float (&sp)[4], const fl
 }
 
 // REGULAR: 16 points in row-major (t rows, s columns) order.
-template <int LC, int V4 = 0>
+template <int LC, int V4 = 0, bool BY_ROW = false>
 __device__ void eval_bspline(float s, float t, int boundary, const int *cvs,
                              const float *src, int stride, int e0, int length,
                              Acc6<LC> &acc) {
@@ -219,7 +219,7 @@ __device__ void eval_bspline(float s, float t, int boundary, const int *cvs,
     int idx[16];
     load_indices<16, LC, V4>(cvs, idx);
     float xc[LC];  // point 5: the patch's (0,0) corner, never a phantom
-    if constexpr (LC == 1) {  // all 16 rows in flight at a time
+    if constexpr (LC == 1 && !BY_ROW) {  // all 16 rows in flight at a time
         float x[16][1];
 #pragma unroll
         for (int j = 0; j < 16; ++j) load_row<1, false>(src, stride, idx[j], e0, length, x[j]);
@@ -572,7 +572,7 @@ __device__ void eval_linear_tri(float s, float t, const int *cvs,
 // OsdEvaluatePatchBasis + gather for one point: normalises (s,t) into the patch, evaluates
 // the basis of `type`, accumulates into acc and returns the derivative scales d1, d2
 // (patchBasis.h:1558-1610).  Returns false for an unknown type.
-template <int LC, bool QUAD_ONLY = false, int V4 = 0>
+template <int LC, bool QUAD_ONLY = false, int V4 = 0, bool BY_ROW = false>
 __device__ bool eval_patch_point(int type, Param p, float s, float t,
                                  const int *cvs, const float *src,
                                  int stride, int e0, int length, Acc6<LC> &acc, float &d1,
@@ -593,14 +593,14 @@ __device__ bool eval_patch_point(int type, Param p, float s, float t,
     }
     if (QUAD_ONLY) {  // Catmull-Clark tables: REGULAR, GREGORY_BASIS, QUADS
         switch (type) {
-            case 6: eval_bspline<LC, V4>(s, t, p.boundary(), cvs, src, stride, e0, length, acc); break;
+            case 6: eval_bspline<LC, V4, BY_ROW>(s, t, p.boundary(), cvs, src, stride, e0, length, acc); break;
             case 9: eval_gregory<LC, V4>(s, t, cvs, src, stride, e0, length, acc); break;
             case 3: eval_linear_quad<LC, V4>(s, t, cvs, src, stride, e0, length, acc); break;
             default: return false;
         }
     } else {
         switch (type) {
-            case 6: eval_bspline<LC, V4>(s, t, p.boundary(), cvs, src, stride, e0, length, acc); break;
+            case 6: eval_bspline<LC, V4, BY_ROW>(s, t, p.boundary(), cvs, src, stride, e0, length, acc); break;
             case 9: eval_gregory<LC, V4>(s, t, cvs, src, stride, e0, length, acc); break;
             case 5: eval_box_tri<LC, V4>(s, t, p.boundary(), cvs, src, stride, e0, length, acc); break;
             case 10: eval_gregory_tri<LC, V4>(s, t, cvs, src, stride, e0, length, acc); break;

@@ -113,6 +113,9 @@ __device__ __forceinline__ void store_packed(float *dst, float *stage, const flo
 // QUAD: Catmull-Clark tables (REGULAR / GREGORY_BASIS / QUADS only): without the Loop and
 // triangle bases the kernel fits 7 blocks per SM for orders 0 and 1 without spills; it is bound by
 // instruction issue (61%), and the packed stores cost it more (79 -> 87 us for 1.7 M coords).
+// PACK: a warp's 32 points at a time, packed outputs stored together.  Not with six outputs of rows
+// that are no quads, where the warp's loop costs registers, whether it packs or not: 2 M Loop points,
+// 2, 3, 5 and 6 floats 116, 151, 350 and 388 us with it, 107, 142, 313 and 362 without.
 // V4: source rows are read as one quad each (patch_basis.cuh; with a row per patch index 4 M Loop
 // points of six outputs take 220 us, copy included, with a row per control point 250).
 template <int LC, int ORDER, bool QUAD = false, int V4 = kAnyRows>
@@ -121,7 +124,7 @@ __global__ void __launch_bounds__(128, LC == 4 ? 4 : (ORDER < 2 && !V4 ? (QUAD ?
     launch_dependents();
     wait_for_primary();
     const PatchArgs a = args_behind_wait<LC, V4>(arg);
-    constexpr bool PACK = LC > 1 && (!QUAD || V4);
+    constexpr bool PACK = LC > 1 && (V4 || (!QUAD && ORDER < 2));
     const int stride = gridDim.x * blockDim.x;
     if constexpr (!PACK) {
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.numCoords; i += stride) {
@@ -177,7 +180,10 @@ __global__ void __launch_bounds__(128, LC == 4 ? 4 : (ORDER < 2 && !V4 ? (QUAD ?
 // G lanes per point, lane l owning primvar elements l, l + G, ...: one source-row fetch is a
 // single coalesced access for the whole group, the accumulators are per element (6 per
 // lane) and no cross-lane reduction is needed.  The basis is evaluated by every lane of the
-// group (cheap for the separable quad-family bases this kernel is used for).
+// group (cheap for the separable quad-family bases this kernel is used for).  P and first derivatives
+// of 6 and more lanes take a REGULAR patch row by row; else its 16 loads are in flight together (2 M
+// points of 5, 8 and 12 floats 1007, 277 and 1012 us so, 944, 266 and 950 row by row; all six outputs
+// of 5 floats 1205 and 1257, P of 8 floats 229 and 234).
 template <int G, int ORDER>
 __global__ void __launch_bounds__(256, 4) k_eval_patches_lanes(const PatchArgs arg) {
     launch_dependents();
@@ -208,8 +214,8 @@ __global__ void __launch_bounds__(256, 4) k_eval_patches_lanes(const PatchArgs a
                 const int type = p.regular() ? arr.regDesc : arr.desc;
                 const int *cvs =
                     a.indices + arr.indexBase + arr.stride * (c.patchIndex - arr.primitiveIdBase);
-                if (!eval_patch_point<1, true>(type, p, c.s, c.t, cvs, a.src, a.srcStride, e,
-                                               a.length, acc, d1, d2))
+                if (!eval_patch_point<1, true, kAnyRows, (ORDER == 1 && G >= 6)>(
+                        type, p, c.s, c.t, cvs, a.src, a.srcStride, e, a.length, acc, d1, d2))
                     acc.zero();
             }
             if (e < a.length) {
