@@ -45,6 +45,10 @@ void scratch_free(void *p, cudaStream_t s);
 // GB300GetDeviceStatus reads and clears; staged kernels record an expired bounded wait there).
 int status_word_address(int **out);
 
+// Whether the `bytes` from p on lie in the one allocation that p points into: they can be read then,
+// whatever they hold.  False where the driver does not know the pointer.  About 0.1 us.
+bool inside_allocation(const void *p, size_t bytes);
+
 // Launches `kern` as the programmatic dependent of the kernel queued before it: it may be started
 // while that one still runs (at once if it called launch_dependents, else when it ends), and calls
 // wait_for_primary before it touches anything that work queued earlier reads or writes.  What it may

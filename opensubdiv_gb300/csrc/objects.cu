@@ -145,7 +145,7 @@ struct PatchSet {
 struct GB300PatchTable {
     int numArrays = 0, numPatches = 0;
     int quadFamily = 0;  // all arrays REGULAR / GREGORY_BASIS / QUADS
-    int numControl = 0;  // largest control index + 1 (rows of the source the table reads)
+    int numControl = 0;  // largest control index + 1 (0: an index is negative)
     int64_t numIndices = 0;
     void *arrays = nullptr, *indices = nullptr, *params = nullptr;
     PatchMapDevice map;
@@ -484,9 +484,12 @@ GB300PatchTable *GB300PatchTableCreate(int numArrays, const void *patchArrays,
     t->numIndices = numIndices;
     t->quadFamily = quad_family(numArrays, arr);
     {
-        int mx = -1;
-        for (int64_t e = 0; e < numIndices; ++e) mx = std::max(mx, patchIndices[e]);
-        t->numControl = mx + 1;
+        int mx = -1, mn = 0;
+        for (int64_t e = 0; e < numIndices; ++e) {
+            mx = std::max(mx, patchIndices[e]);
+            mn = std::min(mn, patchIndices[e]);
+        }
+        t->numControl = mn < 0 ? 0 : mx + 1;
     }
     t->hostArrays.assign(arr, arr + 6 * (size_t)numArrays);
     const char *w = "GB300PatchTableCreate";
@@ -544,11 +547,14 @@ int GB300PatchTableEval(const GB300PatchTable *t, const float *src, float *dst, 
     // and 271 -> 256 over 4.1 M, P and the first derivatives 230 -> 186; P alone 94.5 -> 95.4 of
     // 2 M points: not there).  Catmull-Clark tables read a
     // row with 3 lanes in one access; a padded copy costs them more than it saves (332 us, and
-    // 366 + 24 us over 5.7 M rows).  Not while the stream is captured: the copy's memory would
+    // 366 + 24 us over 5.7 M rows).  The copy reads rows of patches that no
+    // point lies in, which the caller's buffer need not have (a mesh's local points, say): only where
+    // all rows that the table names lie in the buffer's allocation.  Not while the stream is captured: the copy's memory would
     // become part of the caller's graph.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (src && length == 3 && srcStride >= 3 && !t->quadFamily &&
         numPatchCoords >= 65536 && numPatchCoords >= t->numControl && t->numControl > 0 &&
+        inside_allocation(src, ((size_t)(t->numControl - 1) * srcStride + length) * 4) &&
         cudaStreamIsCapturing(s, &capture) == cudaSuccess &&
         capture == cudaStreamCaptureStatusNone) {
         const bool gather = (du || dv || duu || duv || dvv) && t->numIndices <= numPatchCoords;
