@@ -353,11 +353,13 @@ int table_eval(const GB300StencilTable *t, const float *src, float *const *dIn, 
                         "weights",
                         k);
     }
-    if (t->unit.numStencils >= kUnitCall && d[0] && src && units_take(src, srcStride) &&
-        (!units_collect(d[0], st[0]) ||
-         (t->unit.regular && t->unit.numStencils >= kUnitAnyRow)))
-        return eval_stencils_units(t->unit, src, d[0], st[0], length, srcStride, s,
-                                   "GB300StencilTableEval");
+    if (t->unit.numStencils > 0 && d[0] && src && units_take(src, srcStride)) {
+        const UnitRows rows = units_rows(t->unit, d[0], st[0], length,
+                                         (long long)t->numStencils * st[0] * 4, false);
+        if (rows != kUnitNone)
+            return eval_stencils_units(t->unit, rows, src, d[0], st[0], length, srcStride, s,
+                                       "GB300StencilTableEval");
+    }
     if (t->sell.numSlices > 0 && t->sell.idx) {
         const float *sw[6];
         for (int k = 0; k < 6; ++k) sw[k] = d[k] ? t->sell.w[k] : nullptr;

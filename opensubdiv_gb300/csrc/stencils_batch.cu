@@ -1027,15 +1027,26 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
         delete b;
         return nullptr;
     }
-    for (size_t k = 0; k < b->jobs.size(); ++k) {
-        Job &j = b->jobs[k];
-        if (!b->sliced || units[k]->numSlices == 0 ||
-            !units_take(j.src, j.srcStride))
-            continue;
-        j.mode = 3;
-        j.slSz = reinterpret_cast<const int *>(units[k]->slice);
-        j.slIdx = reinterpret_cast<const int *>(units[k]->blob);
-        j.numSlices = units[k]->numSlices;
+    // the jobs that the unit layout takes (units_rows)
+    std::vector<UnitRows> unitRows(b->jobs.size(), kUnitNone);
+    if (b->sliced) {
+        long long bytes = 0, stencils = 0;
+        for (const Job &j : b->jobs) bytes += (long long)j.numStencils * j.dstStride[0] * 4;
+        for (size_t k = 0; k < b->jobs.size(); ++k) {
+            const Job &j = b->jobs[k];
+            if (units[k]->numSlices == 0 || !units_take(j.src, j.srcStride)) continue;
+            unitRows[k] = units_rows(*units[k], j.dst[0], j.dstStride[0], j.length, bytes, true);
+            if (unitRows[k] != kUnitNone) stencils += j.numStencils;
+        }
+        for (size_t k = 0; k < b->jobs.size(); ++k) {
+            Job &j = b->jobs[k];
+            if (stencils < 2 * kUnitTable) unitRows[k] = kUnitNone;
+            if (unitRows[k] == kUnitNone) continue;
+            j.mode = 3;
+            j.slSz = reinterpret_cast<const int *>(units[k]->slice);
+            j.slIdx = reinterpret_cast<const int *>(units[k]->blob);
+            j.numSlices = units[k]->numSlices;
+        }
     }
     // parts: jobs one output 9-12 floats wide over 16-byte aligned rows (stride >= 12) go to
     // the 12-wide launch, jobs at most 4 floats wide over 16-byte aligned rows of a sliced
@@ -1043,8 +1054,8 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
     // largest first)
     {
         const bool sliced = b->sliced;
-        auto part_of = [sliced](const Job &j) {
-            if (j.mode == 3) return units_collect(j.dst[0], j.dstStride[0]) ? 4 : 3;
+        auto part_of = [sliced](const Job &j, UnitRows rows) {
+            if (rows != kUnitNone) return rows == kUnitCollected ? 4 : 3;
             if (j.vw >= 4 && j.length > 8 && j.length <= 12) return 2;
             if (sliced && j.vw >= 4 && j.length <= 4) return 1;
             return 0;
@@ -1052,7 +1063,7 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
         std::vector<Job> pj[kParts];
         std::vector<double> pm[kParts];
         for (size_t k = 0; k < b->jobs.size(); ++k) {
-            const int p = part_of(b->jobs[k]);
+            const int p = part_of(b->jobs[k], unitRows[k]);
             pj[p].push_back(b->jobs[k]);
             pm[p].push_back(b->mean[k]);
         }

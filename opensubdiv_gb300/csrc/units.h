@@ -39,15 +39,12 @@ struct UnitTable {
     int numStencils = 0;
 };
 
-// Tables from kUnitTable stencils on get the layout beside the sliced one.  A batch takes it for all
-// of them: its jobs together fill the SMs.  A single call takes it from kUnitCall on; below, there
-// are too few slices for the SMs' warps (8-wide level-3 rows, against the sliced layout: 131 k
-// stencils 10.3 and 10.3 us, 295 k 12.3 and 14.7 us, 524 k 14.8 and 20.7 us, 1.2 M 29.1 and 39.0 us).
-// Output rows that are not 16-byte aligned are collected, which costs about a third more
-// instructions: a single call takes the layout for them from kUnitAnyRow on, and for regular tables
-// only (5-wide rows: level 3 of quads, 1.2 M stencils 41.5 and 45.2 us, 2.1 M 59.7 and 71.8 us; level
-// 4 of triangles split at random, 1.2 M 50.1 and 39.7 us; in a batch, where the other jobs hide
-// what such a table waits for, they are taken with the rest: 464 and 469 us for the scene).
+// Tables from kUnitTable stencils on get the layout beside the sliced one.  A single call takes it from
+// kUnitCall on; below, there are too few slices for the SMs' warps (8-wide level-3 rows, against the
+// sliced layout: 131 k stencils 10.3 and 10.3 us, 295 k 12.3 and 14.7 us, 524 k 14.8 and 20.7 us, 1.2 M
+// 29.1 and 39.0 us).  A batch's jobs fill the SMs together: it takes the layout for all of them when
+// they have 2 * kUnitTable stencils between them (one job of 75 k stencils, 3- and 12-wide: 13.8 and
+// 12.4 us with it, 12.4 and 10.3 without; of 134 k 13.0 and 12.4, 16.4 and 18.3 without).
 constexpr int kUnitTable = 1 << 16, kUnitCall = 1 << 18, kUnitAnyRow = 3 << 19;
 
 constexpr int kUnitMost = 16;  // stencils per unit
@@ -70,7 +67,13 @@ int build_units(int numStencils, const int *sizes, const int *offsets, const int
 bool units_take(const float *src, int srcStride);
 bool units_collect(const float *dst, int dstStride);
 
-int eval_stencils_units(const UnitTable &t, const float *src, float *dst, int dstStride,
+// How the layout writes `length` floats in rows of `stride` at dst, if it is the better one there: not at
+// all, row by row, or collected.  bytes: the rows of the call, or of all jobs of a batch.
+enum UnitRows { kUnitNone, kUnitByRow, kUnitCollected };
+UnitRows units_rows(const UnitTable &t, const float *dst, int stride, int length, long long bytes,
+                    bool batch);
+
+int eval_stencils_units(const UnitTable &t, UnitRows rows, const float *src, float *dst, int dstStride,
                         int length, int srcStride, cudaStream_t s, const char *who);
 
 }  // namespace gb300
