@@ -885,6 +885,44 @@ int launch_batch(GB300StencilBatch *b, cudaStream_t s, Fork *fork = nullptr) {
     return GB300_OK;
 }
 
+// The same as a graph, captured on first use.
+int launch_graph(GB300StencilBatch *b, cudaStream_t s) {
+    if (!b->graph) {
+        int st = set_smem_attribute();
+        if (st != GB300_OK) return st;
+        if (!b->capture &&
+            (st = check_cuda(cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking),
+                             "batch capture stream")) != GB300_OK)
+            return st;
+        Fork fork;
+        const bool forked = fork.create();  // else one part after the other
+        cudaGraph_t g = nullptr;
+        st = check_cuda(cudaStreamBeginCapture(b->capture, cudaStreamCaptureModeThreadLocal),
+                        "batch graph capture");
+        if (st != GB300_OK) return st;
+        const uint64_t before = g_launches.load();
+        const int lst = launch_batch(b, b->capture, forked ? &fork : nullptr);
+        const cudaError_t ce = cudaStreamEndCapture(b->capture, &g);
+        g_launches.store(before);  // captured, not launched
+        if (lst != GB300_OK) {
+            if (g) cudaGraphDestroy(g);
+            return lst;
+        }
+        if ((st = check_cuda(ce, "batch graph capture")) != GB300_OK) return st;
+        st = check_cuda(cudaGraphInstantiate(&b->graph, g, 0), "batch graph instantiate");
+        cudaGraphDestroy(g);
+        if (st != GB300_OK) {
+            b->graph = nullptr;
+            return st;
+        }
+    }
+    int st = check_cuda(cudaGraphLaunch(b->graph, s), "GB300StencilBatchEvalGraph");
+    if (st != GB300_OK) return st;
+    for (int p = 0; p < kParts; ++p)
+        if (b->partTiles[p]) count_launch();
+    return GB300_OK;
+}
+
 // Jobs whose source rows are unaligned (scalar gathers) and at most 8 floats wide read a
 // padded copy instead: one device buffer for all of them, rows of 8 floats.
 int setup_padding(GB300StencilBatch *b, const std::vector<int> &tableRows, cudaStream_t s) {
@@ -1121,41 +1159,8 @@ int GB300StencilBatchEval(GB300StencilBatch *b, void *stream) {
 
 int GB300StencilBatchEvalGraph(GB300StencilBatch *b, void *stream) {
     if (!b) return fail(GB300_ERR_INVALID_ARGUMENT, "GB300StencilBatchEvalGraph: null batch");
-    cudaStream_t s = as_stream(stream);
-    if (!b->graph) {
-        int st = set_smem_attribute();
-        if (st != GB300_OK) return st;
-        if (!b->capture &&
-            (st = check_cuda(cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking),
-                             "batch capture stream")) != GB300_OK)
-            return st;
-        Fork fork;
-        const bool forked = fork.create();  // else one part after the other
-        cudaGraph_t g = nullptr;
-        st = check_cuda(cudaStreamBeginCapture(b->capture, cudaStreamCaptureModeThreadLocal),
-                        "batch graph capture");
-        if (st != GB300_OK) return st;
-        const uint64_t before = g_launches.load();
-        const int lst = launch_batch(b, b->capture, forked ? &fork : nullptr);
-        const cudaError_t ce = cudaStreamEndCapture(b->capture, &g);
-        g_launches.store(before);  // captured, not launched
-        if (lst != GB300_OK) {
-            if (g) cudaGraphDestroy(g);
-            return lst;
-        }
-        if ((st = check_cuda(ce, "batch graph capture")) != GB300_OK) return st;
-        st = check_cuda(cudaGraphInstantiate(&b->graph, g, 0), "batch graph instantiate");
-        cudaGraphDestroy(g);
-        if (st != GB300_OK) {
-            b->graph = nullptr;
-            return st;
-        }
-    }
-    int st = check_cuda(cudaGraphLaunch(b->graph, s), "GB300StencilBatchEvalGraph");
-    if (st != GB300_OK) return st;
-    for (int p = 0; p < kParts; ++p)
-        if (b->partTiles[p]) count_launch();
-    return ok();
+    const int st = launch_graph(b, as_stream(stream));
+    return st != GB300_OK ? st : ok();
 }
 
 int GB300StencilBatchGetDeviceStatus(GB300StencilBatch *b, int *status) {
@@ -1205,10 +1210,15 @@ int GB300StencilBatchTune(GB300StencilBatch *b, int iterations, void *stream) {
                 if (b->sliced && (ts != tiles[0] || th != thresholds[0])) continue;
                 b->cfg = Config{ts, c, th, dyn};
                 if ((st = upload_plan(b, s)) != GB300_OK) goto done;
-                if ((st = launch_batch(b, s)) != GB300_OK) goto done;  // warm-up
+                // both ways of running it, once to warm up: a graph's parts are branches
+                b->drop_graph();
+                if ((st = launch_batch(b, s)) != GB300_OK) goto done;
+                if ((st = launch_graph(b, s)) != GB300_OK) goto done;
                 cudaEventRecord(e0, s);
                 for (int k = 0; k < iterations; ++k)
                     if ((st = launch_batch(b, s)) != GB300_OK) goto done;
+                for (int k = 0; k < iterations; ++k)
+                    if ((st = launch_graph(b, s)) != GB300_OK) goto done;
                 cudaEventRecord(e1, s);
                 cudaEventSynchronize(e1);
                 float ms = 0.0f;
@@ -1221,6 +1231,7 @@ int GB300StencilBatchTune(GB300StencilBatch *b, int iterations, void *stream) {
 done:
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    b->drop_graph();
     b->cfg = best;
     const int rb = upload_plan(b, s);
     if (st != GB300_OK) return st;
