@@ -90,88 +90,36 @@ __device__ __forceinline__ void eval_point(const PatchArgs &a, const Coord &c, i
     scale[3] = scale[4] = scale[5] = d2;
 }
 
-// One output of the warp's 32 points from point `first` on, whose rows
-// follow one another (stride = length = LC): written through shared memory, so that every store
-// covers whole sectors (by its thread, a row of 3 floats takes 3 stores to another
-// sector each: 29.1 M sectors written for 4 M points, where the outputs have 9.0 M).
-template <int LC>
-__device__ __forceinline__ void store_packed(float *dst, float *stage, const float (&v)[LC],
-                                             int first, int n, int lane) {
-    __syncwarp();
-#pragma unroll
-    for (int m = 0; m < LC; ++m) stage[lane * LC + m] = v[m];
-    __syncwarp();
-    float *out = dst + (size_t)first * LC;
-    const int count = (n - first < 32 ? n - first : 32) * LC;
-#pragma unroll
-    for (int m = 0; m < LC; ++m)
-        if (lane + 32 * m < count) st_stream(out + lane + 32 * m, stage[lane + 32 * m]);
-}
-
 // 5 resident blocks per SM where the registers allow it without spills (0.2847 vs 0.2908 ms
 // for 4 M Loop points at LC = 3; LC = 4 would spill)
 // QUAD: Catmull-Clark tables (REGULAR / GREGORY_BASIS / QUADS only): without the Loop and
-// triangle bases the kernel fits 7 blocks per SM for orders 0 and 1 without spills; it is bound by
-// instruction issue (61%), and the packed stores cost it more (79 -> 87 us for 1.7 M coords).
-// PACK: a warp's 32 points at a time, packed outputs stored together.  Not with six outputs of rows
-// that are no quads, where the warp's loop costs registers, whether it packs or not: 2 M Loop points,
-// 2, 3, 5 and 6 floats 116, 151, 350 and 388 us with it, 107, 142, 313 and 362 without.
+// triangle bases the kernel fits 7 blocks per SM for orders 0 and 1 without spills.
+// Outputs are stored by their threads: collected through shared memory, whole sectors a store, they
+// take the warp a loop of its own and the registers for it (4 M Loop points of xyz, 71 k rows: P 164
+// and 173 us, with first derivatives 170 and 181, all six 199 and 211; points in patch order, 2.9 M
+// coords of a tessellation, 132 and 154).
 // V4: source rows are read as one quad each (patch_basis.cuh; with a row per patch index 4 M Loop
-// points of six outputs take 220 us, copy included, with a row per control point 250).
+// points of six outputs take 205 us, copy included, with a row per control point 231, in place 293).
 template <int LC, int ORDER, bool QUAD = false, int V4 = kAnyRows>
 __global__ void __launch_bounds__(128, LC == 4 ? 4 : (ORDER < 2 && !V4 ? (QUAD ? 7 : 6) : 5))
     k_eval_patches(const PatchArgs arg) {
     launch_dependents();
     wait_for_primary();
     const PatchArgs a = args_behind_wait<LC, V4>(arg);
-    constexpr bool PACK = LC > 1 && (V4 || (!QUAD && ORDER < 2));
     const int stride = gridDim.x * blockDim.x;
-    if constexpr (!PACK) {
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.numCoords; i += stride) {
-            const Coord c = load_coord(a.coords + i);
-            for (int e0 = 0; e0 < a.length; e0 += LC) {
-                Acc6<LC> acc;
-                float scale[6];
-                eval_point<LC, QUAD, V4>(a, c, e0, acc, scale);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.numCoords; i += stride) {
+        const Coord c = load_coord(a.coords + i);
+        for (int e0 = 0; e0 < a.length; e0 += LC) {
+            Acc6<LC> acc;
+            float scale[6];
+            eval_point<LC, QUAD, V4>(a, c, e0, acc, scale);
 #pragma unroll
-                for (int k = 0; k <= last_output(ORDER); ++k) {
-                    if (!(a.active & (1 << k))) continue;
-                    float *out = a.dst[k] + (size_t)i * a.dstStride[k] + e0;
+            for (int k = 0; k <= last_output(ORDER); ++k) {
+                if (!(a.active & (1 << k))) continue;
+                float *out = a.dst[k] + (size_t)i * a.dstStride[k] + e0;
 #pragma unroll
-                    for (int m = 0; m < LC; ++m)
-                        if (e0 + m < a.length) st_stream(out + m, acc.v[k][m] * scale[k]);
-                }
-            }
-        }
-    } else {
-        // a warp's 32 points at a time, the last ones with idle lanes
-        __shared__ float stage[4][32 * LC];
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        for (int first = blockIdx.x * blockDim.x + 32 * warp; first < a.numCoords;
-             first += stride) {
-            const int i = first + lane;
-            const bool on = i < a.numCoords;
-            Coord c{-1, 0, 0, 0.0f, 0.0f};
-            if (on) c = load_coord(a.coords + i);
-            for (int e0 = 0; e0 < a.length; e0 += LC) {
-                Acc6<LC> acc;
-                float scale[6];
-                eval_point<LC, QUAD, V4>(a, c, e0, acc, scale);
-#pragma unroll
-                for (int k = 0; k <= last_output(ORDER); ++k) {
-                    if (!(a.active & (1 << k))) continue;
-                    float v[LC];
-#pragma unroll
-                    for (int m = 0; m < LC; ++m) v[m] = acc.v[k][m] * scale[k];
-                    if (a.length == LC && a.dstStride[k] == LC) {
-                        store_packed<LC>(a.dst[k], stage[warp], v, first, a.numCoords, lane);
-                    } else if (on) {
-                        float *out = a.dst[k] + (size_t)i * a.dstStride[k] + e0;
-#pragma unroll
-                        for (int m = 0; m < LC; ++m)
-                            if (e0 + m < a.length) st_stream(out + m, v[m]);
-                    }
-                }
+                for (int m = 0; m < LC; ++m)
+                    if (e0 + m < a.length) st_stream(out + m, acc.v[k][m] * scale[k]);
             }
         }
     }
