@@ -541,25 +541,33 @@ int GB300PatchTableEval(const GB300PatchTable *t, const float *src, float *dst, 
     float *d[6] = {dst, du, dv, duu, duv, dvv};
     const int st[6] = {dstStride, duStride, dvStride, duuStride, duvStride, dvvStride};
     cudaStream_t s = as_stream(stream);
-    // Loop tables are evaluated one point per thread, 13 rows each: rows of 3 floats are read from
-    // a copy padded to 4 (one load per row), as soon as there are more points than rows to copy
-    // (4 M points, 226 k rows: 298 us, and 238 + 4 us with the copy).  With derivatives and as many
-    // points as patch indices the copy has a row per index, so that a patch's rows follow one another
-    // and no index is read (4 M points, copy included: six outputs 250 -> 220 us over 1.0 M indices
-    // and 271 -> 256 over 4.1 M, P and the first derivatives 230 -> 186; P alone 94.5 -> 95.4 of
-    // 2 M points: not there).  Catmull-Clark tables read a
-    // row with 3 lanes in one access; a padded copy costs them more than it saves (332 us, and
-    // 366 + 24 us over 5.7 M rows).  The copy reads rows of patches that no
-    // point lies in, which the caller's buffer need not have (a mesh's local points, say): only where
-    // all rows that the table names lie in the buffer's allocation.  Not while the stream is captured: the copy's memory would
-    // become part of the caller's graph.
+    // Loop tables are evaluated one point per thread, 13 rows each: many points read rows of 3 floats
+    // from a copy padded to 4, one load per row; with derivatives and rows that outgrow L1 the copy has
+    // a row per patch index, so that a patch's rows follow one another and no index is read.  us,
+    // copy included, of scattered points, a row per index / per control point / in place:
+    //   2.4 k rows:  0.14 M points, P 12.9/11.5/9.1; 0.27 M 14.2/14.2/12.7; 1.0 M, P and first
+    //                derivatives 44/41/42, six outputs 52/48/51
+    //   28 k rows:   0.14 M points, P 11.7/11.3/12.1; 0.27 M 16.1/16.0/18.5; 4.0 M, P and first
+    //                derivatives 168/175/237, six outputs 193/189/242
+    //   226 k rows:  4.0 M points, P 190/191/249, P and first derivatives 174/223/286, six 205/231/293
+    // so from 2^18 points on, or 3/4 of them over more than 8,192 rows, and with at least as many points
+    // as rows to copy.  Points in the order of their patches find a patch's rows in L1 as they are (4.0 M,
+    // 226 k rows: P 94 and 87 us in place, P and first derivatives 116 and 129, six 156 and 178);
+    // GB300TessellationEvaluate is for those.  Catmull-Clark tables read a row with 3 lanes in one
+    // access; a padded copy costs them more than it saves (332 us, and 366 + 24 us over 5.7 M rows).
+    // The copy reads rows of patches that no point lies in, which the caller's buffer need not have
+    // (a mesh's local points, say): only where all rows that the table names lie in the buffer's
+    // allocation.  Not while the stream is captured: the copy's memory would become part of the caller's
+    // graph.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (src && length == 3 && srcStride >= 3 && !t->quadFamily &&
-        numPatchCoords >= 65536 && numPatchCoords >= t->numControl && t->numControl > 0 &&
+        numPatchCoords >= (t->numControl > 8192 ? 3 << 16 : 1 << 18) &&
+        numPatchCoords >= t->numControl && t->numControl > 0 &&
         inside_allocation(src, ((size_t)(t->numControl - 1) * srcStride + length) * 4) &&
         cudaStreamIsCapturing(s, &capture) == cudaSuccess &&
         capture == cudaStreamCaptureStatusNone) {
-        const bool gather = (du || dv || duu || duv || dvv) && t->numIndices <= numPatchCoords;
+        const bool gather = (du || dv || duu || duv || dvv) && t->numControl >= 1 << 15 &&
+                            t->numIndices <= numPatchCoords;
         const size_t rows = gather ? (size_t)t->numIndices : (size_t)t->numControl;
         float *padded = nullptr;
         if (scratch_alloc((void **)&padded, rows * 16, s, who) == GB300_OK) {

@@ -86,8 +86,11 @@ int eval_stencils(const float *, float *const *, const int *, const float *const
 int eval_stencils_sell(const SellTable &, const float *, float *const *, const int *,
                        const float *const *, int, int, cudaStream_t,
                        const char *) { return GB300_OK; }
-int eval_stencils_units(const UnitTable &, const float *, float *, int, int, int, cudaStream_t,
-                        const char *) { return GB300_OK; }
+UnitRows units_rows(const UnitTable &, const float *, int, int, long long, bool) {
+    return kUnitNone;
+}
+int eval_stencils_units(const UnitTable &, UnitRows, const float *, float *, int, int, int,
+                        cudaStream_t, const char *) { return GB300_OK; }
 int find_patches(const PatchMapDevice &, int, const int *, const float *, const float *, void *,
                  cudaStream_t) { return GB300_OK; }
 int tess_factors(const void *, int, const int *, const void *, int, const float *, int,
@@ -115,36 +118,38 @@ int eval_patches(const float *src, float *const *, const int *, int, int, int, c
 }  // namespace gb300
 
 int main() {
-    // two Loop patches of 12 points: the second one names rows up to 999
+    // two Loop patches of 12 points: the second one names rows up to rows - 1, few (a copy of the rows)
+    // or many (with derivatives a row per index)
     const int arrays[6] = {5, 5, 2, 0, 12, 0};
     int indices[24], params[6] = {};
-    for (int j = 0; j < 24; ++j) indices[j] = j < 12 ? j : 999 - (j - 12);
-    static float buffer[4000];
-    const int n = 70000;
+    static float buffer[4 * 40000];
+    const int n = 1 << 18;
     for (int stride = 3; stride <= 4; ++stride)
-        for (int more = 0; more < 2; ++more)  // P alone, and with derivatives (a row per index)
+        for (int more = 0; more < 4; ++more)  // P alone, and with derivatives; few rows, and many
             for (int offset = 0; offset < 2; ++offset)
                 for (int negative = 0; negative < 2; ++negative) {
-                    indices[23] = negative ? -1 : 988;
+                    const int rows = more < 2 ? 1000 : 40000;
+                    for (int j = 0; j < 24; ++j) indices[j] = j < 12 ? j : rows - 1 - (j - 12);
+                    if (negative) indices[23] = -1;
                     GB300PatchTable *t =
                         GB300PatchTableCreate(1, arrays, 24, indices, 2, params, 1, nullptr);
                     if (!t) return printf("no table\n"), 1;
-                    const size_t need = (999 * (size_t)stride + 3 + offset) * 4;
+                    const size_t need = ((rows - 1) * (size_t)stride + 3 + offset) * 4;
                     for (int state = 0; state < 4; ++state) {
                         // the whole buffer, a float less, one patch's rows, an unknown pointer
                         g_known = state < 3;
                         g_start = (uintptr_t)buffer;
                         g_size = state == 0 ? need : state == 1 ? need - 4 : 12 * stride * 4;
                         g_copied = g_evaluated = 0;
-                        float *du = more ? buffer : nullptr;
+                        float *du = more & 1 ? buffer : nullptr;
                         const int st = GB300PatchTableEval(t, buffer + offset, buffer, du, nullptr,
                                                            nullptr, nullptr, nullptr, 3, stride, 3,
                                                            3, 3, 3, 3, 3, n, buffer, nullptr);
                         const int want = state == 0 && !negative;
                         if (st != GB300_OK || g_evaluated != 1 || g_copied != want ||
                             (g_source == buffer + offset) == (want == 1))
-                            return printf("stride %d more %d offset %d negative %d state %d: "
-                                          "status %d, %d copies\n", stride, more, offset, negative,
+                            return printf("rows %d stride %d more %d offset %d negative %d state %d: "
+                                          "status %d, %d copies\n", rows, stride, more, offset, negative,
                                           state, st, g_copied), 1;
                     }
                     GB300PatchTableDestroy(t);

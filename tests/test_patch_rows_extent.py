@@ -27,9 +27,9 @@ def test_the_copy_stays_in_the_buffer(tmp_path):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("outputs", [1, 6])
-def test_rows_that_no_point_needs_may_be_missing(outputs):
-    """Two instances of a Loop mesh, the points all in the first, whose rows are all that the buffer
+@pytest.mark.parametrize("outputs,copies", [(1, 2), (6, 2), (6, 15)])
+def test_rows_that_no_point_needs_may_be_missing(outputs, copies):
+    """Instances of a Loop mesh, the points all in the first, whose rows are all that the buffer
     has: the bits of calls of fewer points, which read the rows of their patches only."""
     torch = torch_cuda()
     from opensubdiv_gb300 import workloads
@@ -39,9 +39,9 @@ def test_rows_that_no_point_needs_may_be_missing(outputs):
         z = {k: f[k] for k in f.files}
     if "num_ptex" not in z:
         z["num_ptex"] = z["ptex_offsets"][-1]
-    arrays, indices, params, _, ptex, tri = workloads.instanced_patch_table(z, 2)
+    arrays, indices, params, _, ptex, tri = workloads.instanced_patch_table(z, copies)
     table = GB300PatchTable.Create(arrays, indices, params, tri)
-    n = 65536 + 33
+    n = (1 << 18) + 33
     rng = np.random.default_rng(9)
     face = rng.integers(0, int(z["num_ptex"]), n).astype(np.int32)
     u, v = rng.random(n, np.float32), rng.random(n, np.float32)
@@ -54,7 +54,7 @@ def test_rows_that_no_point_needs_may_be_missing(outputs):
     buffer = GB300VertexBuffer.Create(3, rows.shape[0])
     buffer.UpdateData(rows, 0, rows.shape[0])
     d, got = BD(0, 3, 3), []
-    for step in (n, 40000):
+    for step in (n, 100000):
         out = [torch.zeros((n, 3), device="cuda") for _ in range(outputs)]
         for lo in range(0, n, step):
             m, kw = min(step, n - lo), {}
