@@ -6,8 +6,8 @@
 // (bit 31 set, bit 30 leaf, bits 0..29 node or handle index).  Quad tables walk in float:
 // every step subtracts a power of two `median` from a value in [median, 2*median], which is
 // exact (Sterbenz), so the float walk takes the reference's double-precision decisions.
-// Triangle tables walk the same way and form only their u + v tests in double, as the
-// reference rounds them.
+// Triangle tables walk the same way; their u + v tests compare the exact sums, which decide as the
+// reference's rounded double sums do.
 #include "common.cuh"
 #include "patchmap.h"
 #include "patchmap_walk.cuh"
@@ -134,11 +134,16 @@ struct FindArgs {
 // written by their threads (5 stores, 20 bytes apart) they took 10.6 M sector writes for 4 M queries
 // instead of 3.7 M.  4 M queries of a quad tree: 69.5 us, 52.4 us with these stores, 44 us with
 // handles computed from the leaf; of a triangle tree 74.8 us, 37.5 us with both and the sums
-// compared without the FP64 pipe (patchmap_walk.cuh).
+// compared without the FP64 pipe (patchmap_walk.cuh).  Of a small table neither pays (direct): its
+// handles stay in L1, and what is left is instructions (4 M queries of 6,107 patches 33 us, 36 with
+// these stores, 39 with both; of 24 k patches 42, 39 and 40).
+constexpr int kSmallMap = 1 << 14;
+
+template <bool DIRECT>
 __global__ void __launch_bounds__(256) k_find_patches(const FindArgs a) {
     launch_dependents();
     wait_for_primary();
-    __shared__ int stage[8][32 * 5];
+    __shared__ int stage[DIRECT ? 1 : 8][32 * 5];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int stride = gridDim.x * blockDim.x;
     for (int first = blockIdx.x * blockDim.x + 32 * warp; first < a.n; first += stride) {
@@ -146,13 +151,14 @@ __global__ void __launch_bounds__(256) k_find_patches(const FindArgs a) {
         if (i < a.n) {
             const float fu = a.u[i], fv = a.v[i];
             const int4 h = patch_map_find(a.map, a.faces[i], fu, fv);
-            int *o = stage[warp] + 5 * lane;
+            int *o = DIRECT ? a.out + 5 * (size_t)i : stage[warp] + 5 * lane;
             o[0] = h.x;
             o[1] = h.y;
             o[2] = h.z;
             o[3] = __float_as_int(fu);
             o[4] = __float_as_int(fv);
         }
+        if (DIRECT) continue;
         __syncwarp();
         const int count = 5 * (a.n - first < 32 ? a.n - first : 32);
         int *out = a.out + 5 * (size_t)first;
@@ -172,8 +178,6 @@ PatchMapView view_of(const PatchMapDevice &m) {
     v.maxDepth = m.maxDepth;
     v.triangular = m.triangular;
     v.numPatches = m.numPatches;
-    v.numArrays = m.numArrays;
-    for (int a = 0; a < kMapArrays; ++a) v.first[a] = m.first[a], v.step[a] = m.step[a];
     return v;
 }
 
@@ -189,10 +193,16 @@ int find_patches(const PatchMapDevice &m, int n, const int *faces, const float *
     a.u = u;
     a.v = v;
     a.out = (int *)coordsOut;
+    const bool direct = m.numPatches < kSmallMap;
+    if (!direct) {
+        a.map.numArrays = m.numArrays;
+        for (int k = 0; k < kMapArrays; ++k) a.map.first[k] = m.first[k], a.map.step[k] = m.step[k];
+    }
     const int threads = 256;
     long long blocks = ((long long)n + threads - 1) / threads;
     long long cap = (long long)num_sms() * 16;
-    launch_kernel(k_find_patches, (int)(blocks < cap ? blocks : cap), threads, 0, s, a);
+    launch_kernel(direct ? k_find_patches<true> : k_find_patches<false>,
+                  (int)(blocks < cap ? blocks : cap), threads, 0, s, a);
     return check_launch("FindPatches");
 }
 

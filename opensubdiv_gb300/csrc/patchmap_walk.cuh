@@ -19,8 +19,8 @@ struct PatchMapView {
     const int4 *handles;
     int minFace, maxFace, maxDepth, triangular, numPatches;
     // first patch and indices per patch of each patch array, for tables of at most kMapArrays
-    // (numArrays 0: more): a handle is then computed from the leaf instead of loaded (one random
-    // 16-byte read less per query, out of 23 MB for 1.4 M patches)
+    // (numArrays 0: loaded): a handle is then computed from the leaf instead of loaded (one random
+    // 16-byte read less per query, out of 23 MB for 1.4 M patches; small tables' stay in L1)
     int numArrays = 0;
     int first[kMapArrays] = {}, step[kMapArrays] = {};
 };
