@@ -331,20 +331,6 @@ __global__ void __launch_bounds__(128, 8) k_tess_generate(const GenArgs a, int f
     }
 }
 
-// The 32 coords from i0 on of a face of nc coords, located, written through shared memory (`stage`:
-// 160 words of the warp): whole sectors of the 20-byte records.
-__device__ __forceinline__ void locate_coords(const GenArgs &a, int N, int ptex0, float2 uv, int i0,
-                                              int nc, int64_t c0, int *stage, int lane) {
-    if (i0 + lane < nc) locate_coord(a, N, ptex0, uv.x, uv.y, stage + 5 * lane);
-    __syncwarp();
-    const int words = 5 * min(32, nc - i0);
-    int *out = a.patchCoords + 5 * (c0 + i0);
-#pragma unroll
-    for (int m = 0; m < 5; ++m)
-        if (lane + 32 * m < words) out[lane + 32 * m] = stage[lane + 32 * m];
-    __syncwarp();
-}
-
 // A face's nf facets at `from` (facets `step` words apart) moved by `delta` into its slice at
 // facet f0 of the output: word by word where both are packed, so that neighbouring lanes write
 // neighbouring words.
@@ -379,25 +365,29 @@ __device__ __forceinline__ void move_facets(const GenArgs &a, const int *from, i
 
 // One warp per face: copies a shared pattern, or the slice of the face that owns its pattern,
 // into its own (coords as float2 pairs), and locates every coord of the face on the patch table.
+// The records of located coords are stored by their lanes and their handles loaded: neighbouring coords
+// lie in few patches, and most faces have fewer coords than a warp lanes (rate 5, 138 k quads: 81 us so,
+// 100 with the stores and handles of k_find_patches; rate 3, 55 k quads 26 and 30).  Small faces are
+// bound by the latency of a face's first loads, which are asked for together, and by the last faces of
+// a warp: 16 CTAs per SM, of which 8 are resident (rate 2, 138 k quads 56 us with the loads one after
+// another and 8 CTAs, 49 so, 33 and 29 without patches).
 template <int FS>
-__global__ void __launch_bounds__(256) k_tess_finish(const GenArgs a) {
+__global__ void __launch_bounds__(256, 8) k_tess_finish(const GenArgs a) {
     launch_dependents();
     wait_for_primary();
-    __shared__ int stages[8][160];
     const int lane = threadIdx.x & 31;
-    int *stage = stages[threadIdx.x >> 5];
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int f = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; f < a.numFaces; f += warps) {
-        const int64_t c0 = a.co[f];
-        const int nc = (int)(a.co[f + 1] - c0);
-        if (nc == 0) continue;
         const int N = a.faceSizes[f];
+        const int64_t c0 = a.co[f], f0 = a.fo[f];
+        const int nc = (int)(a.co[f + 1] - c0), nf = (int)(a.fo[f + 1] - f0);
+        const int ptex0 = a.locate ? (int)a.po[f] : 0;
+        if (nc == 0) continue;
         const bool sh = uses_shared(a, N);
         const int own = sh ? f : owner_of(a, f);
         const bool copy = sh || own != f;
         if (!copy && !a.locate) continue;
         const int k = N - kFirstShared;
-        const int ptex0 = a.locate ? (int)a.po[f] : 0;
         const int64_t s0 = sh ? 0 : a.co[own];
         const float *from =
             sh ? a.patCoords + 2 * (int64_t)a.patC[k] : a.coords + s0 * a.coordStride;
@@ -419,11 +409,10 @@ __global__ void __launch_bounds__(256) k_tess_finish(const GenArgs a) {
                     }
                 }
             }
-            if (a.locate) locate_coords(a, N, ptex0, uv, i0, nc, c0, stage, lane);
+            if (a.locate && i < nc)
+                locate_coord(a, N, ptex0, uv.x, uv.y, a.patchCoords + 5 * (c0 + i));
         }
         if (!copy) continue;
-        const int64_t f0 = a.fo[f];
-        const int nf = (int)(a.fo[f + 1] - f0);
         if (sh)
             move_facets<FS>(a, a.patFacets + FS * a.patF[k], FS, f0, nf,
                             a.offsetIndices ? (int)c0 : 0, lane);
@@ -1135,7 +1124,7 @@ extern "C" int GB300TessellationGenerate(
         st = check_launch(who);
     }
     if (st == GB300_OK && (a.shared || a.locate || a.dedupe)) {
-        const int blocks = grid_for((long long)numFaces * 32, 256, 8);
+        const int blocks = grid_for((long long)numFaces * 32, 256, 16);
         if (o.fs == 4)
             launch_kernel(k_tess_finish<4>, blocks, 256, 0, s, a);
         else
