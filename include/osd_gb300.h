@@ -129,7 +129,10 @@ typedef struct GB300StencilTable GB300StencilTable;
  * same source rows together.  The Get*Buffer arrays hold that layout.  The table also keeps a
  * second, evaluation-only copy built on the device (32-stencil slices stored entry-major, in
  * locality order), which GB300StencilTableEval reads; it takes about as much device memory
- * as the Get*Buffer arrays. */
+ * as the Get*Buffer arrays.  A table of one weight array with 65,536 stencils or more keeps a third
+ * one, in which stencils with the same control indices are evaluated together (a quarter to two
+ * thirds of the arrays' size), for large tables and for batches; without memory for it the
+ * table does without. */
 GB300StencilTable *GB300StencilTableCreate(int numStencils, int64_t nnz, const int *sizes,
                                            const int *offsets, const int *indices,
                                            const float *weights, const float *duWeights,
@@ -228,7 +231,11 @@ int GB300PatchTableGetNumPatches(const GB300PatchTable *table);
 int GB300PatchTableFindPatches(const GB300PatchTable *table, int n, const int *faces,
                                const float *u, const float *v, void *coordsOut, void *stream);
 
-/* EvalPatches against a device table (CudaEvaluator::EvalPatches template form). */
+/* EvalPatches against a device table (CudaEvaluator::EvalPatches template form).  Points may come in
+ * any order; points in the order of their patches (a tessellation's) are read faster by
+ * GB300TessellationEvaluate.  For many points of a Loop table the call may read every source row that
+ * the table names, not only those of the points' patches, where the buffer's allocation has them
+ * all; their values do not matter. */
 int GB300PatchTableEval(const GB300PatchTable *table, const float *src, float *dst, float *du,
                         float *dv, float *duu, float *duv, float *dvv, int length,
                         int srcStride, int dstStride, int duStride, int dvStride,
@@ -469,8 +476,8 @@ int GB300VertexBufferGetNumVertices(const GB300VertexBuffer *buffer);
 
 /* ---- batched EvalStencils (no counterpart in the reference) ------------------------------ */
 
-/* A batch evaluates many meshes' device stencil tables in ONE persistent launch, instead of one
- * GB300StencilTableEval (CudaEvaluator::EvalStencils, osd/cudaEvaluator.h:125-142) per mesh:
+/* A batch evaluates many meshes' device stencil tables in a few persistent launches (one for each
+ * kind of rows that its jobs have, five at most), instead of one GB300StencilTableEval (CudaEvaluator::EvalStencils, osd/cudaEvaluator.h:125-142) per mesh:
  * job i computes dst[i][k*dstStride[i] + e] = sum_j w_j * src[i][idx_j*srcStride[i] + e] for
  * every stencil k of tables[i] and element e < length[i] (pointers already include the
  * BufferDescriptor offset, as in the raw EvalStencils forms).  Results are those of the
@@ -481,26 +488,28 @@ typedef struct GB300StencilBatch GB300StencilBatch;
 
 /* Builds the job table and the tile prefix on the device (synchronous on `stream`).  When
  * every table has its sliced evaluation layout (tables from GB300StencilTableCreate and the
- * factories), the batch reads those: tiles of 8 slices, one warp per 32-stencil slice;
- * otherwise the Far-layout arrays.  Jobs whose source rows are unaligned (no 16-byte vector
- * loads) and at most 8 floats wide get a device buffer for a padded copy of their source
- * (rows of 8 floats), refreshed by every evaluation.  Uses the tuned configuration cached for batches with the same work histogram,
- * if any.  Returns NULL on failure (error string set). */
+ * factories), the batch reads those: tiles of 8 slices, one warp per 32-stencil slice, and the
+ * unit layout of large tables; otherwise the Far-layout arrays.  Jobs whose source rows are
+ * unaligned (no 16-byte vector loads) and at most 16 floats wide get a device buffer for a padded
+ * copy of their source (rows of 4, 8, 12 or 16 floats), refreshed by every evaluation.  Uses the
+ * tuned configuration cached for batches with the same work histogram, if any.  Returns NULL on failure (error string set). */
 GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const *tables,
                                            const float *const *src, float *const *dst,
                                            const int *length, const int *srcStride,
                                            const int *dstStride, void *stream);
 void GB300StencilBatchDestroy(GB300StencilBatch *batch);
-/* One evaluation of every job: a counter reset and one kernel on `stream`. */
+/* One evaluation of every job on `stream`: the padded copies, then one to five kernels and the resets
+ * of their counters, one after the other. */
 int GB300StencilBatchEval(GB300StencilBatch *batch, void *stream);
 /* The same, replayed from a CUDA graph captured on the first call (on a private stream) and
- * launched on `stream`.  The graph is dropped and recaptured after GB300StencilBatchTune. */
+ * launched on `stream`, the kernels side by side.  The graph is dropped and recaptured after
+ * GB300StencilBatchTune. */
 int GB300StencilBatchEvalGraph(GB300StencilBatch *batch, void *stream);
 /* Autotuner: times each candidate (stencils per tile, CTAs per SM (1-3, capped by what the
  * kernel keeps resident), mean stencil size above which a job switches to one warp per
  * stencil, tiles claimed from a work counter or assigned round-robin; sliced batches only try
- * the CTA counts and the claim order) over `iterations` evaluations on the batch itself, keeps the fastest, and
- * caches it for later batches with the same histogram of work over (stencil size, job size,
+ * the CTA counts and the claim order) over `iterations` evaluations on the batch itself, by Eval and
+ * by EvalGraph, keeps the one with the least sum, and caches it for later batches with the same histogram of work over (stencil size, job size,
  * primvar width) classes.  Writes the outputs as Eval does. */
 int GB300StencilBatchTune(GB300StencilBatch *batch, int iterations, void *stream);
 int GB300StencilBatchGetConfig(const GB300StencilBatch *batch, int *tileStencils,

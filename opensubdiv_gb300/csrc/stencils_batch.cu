@@ -1,4 +1,5 @@
-// Batched EvalStencils: many meshes of uneven sizes in ONE persistent launch.
+// Batched EvalStencils: many meshes of uneven sizes in a few persistent launches, one for each kind of
+// rows that they have (five at most).
 //
 // A launch is a device job table (one job per mesh: its stencil table arrays, source and
 // destination with the descriptor offset applied, primvar length and strides) plus the prefix

@@ -431,7 +431,7 @@ __device__ __forceinline__ void store_cols(const SellArgs &a, int o, int row, in
 // Three CTAs per SM for one output (72 registers, 53 KB of ring each: the gathers are
 // latency-bound and the smaller carve-out leaves more L1 for source rows; 0.267 -> 0.238 ms on
 // the refine pass, 12-wide rows 0.372 -> 0.356 ms), and for 3 outputs over rows of up to 4
-// floats; two otherwise (more would spill), one for 6 outputs.
+// floats; two otherwise (more would spill), one for 6 outputs of wider rows.
 template <int NW, int VW>
 __global__ void __launch_bounds__(kThreads, NW == 1 || (NW == 3 && VW == kNarrow) ? 3 : NW >= 6 && VW != kNarrow ? 1 : 2)
     k_stencils_sell(const SellArgs a) {

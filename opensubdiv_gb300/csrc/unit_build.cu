@@ -366,8 +366,11 @@ int build_units(int n, const int *sizes, const int *offsets, const int *indices,
         tmp.drop(q);
     };
     // Larger units read fewer source rows and hold fewer index lists; smaller ones make more
-    // slices.  8.6 M stencils (8-wide rows): 110 us with 16, 132 with 7; 0.5 M and 1.0 M Loop
-    // stencils: 36.8 us with 16, 28.9 with 7 (12-wide: 50.9, 39.7).
+    // slices, which a small table lacks, and wait for fewer weights where slices are not uniform.
+    // us with 8 and 16: level 3 of quads, 8-wide rows, 0.3 M stencils 8.8 and 11.8, 2.1 M 34.9
+    // and 33.0, 4.3 M 62 and 57, 5.2 M 76 and 68, 8.6 M 120 and 104 (12-wide 227 and 240, xyz 122 and
+    // 132); level 4, 8.6 M 123 and 120; irregular tables, 8-wide, 0.65 M 17.7 and 14.7, 1.9 M 42.8
+    // and 46.1, 4.1 M 81 and 87, 8.5 M 156 and 169; Loop, level 3, 1.3 M 27.6 and 33.2, 8.0 M 139 and 136.
     const int most = n >= (4 << 20) ? kUnitMost : kUnitMost / 2;
 
     // stencils in locality order, equal lists together

@@ -355,7 +355,7 @@ class GB300StencilTableFactory:
 
 
 class GB300StencilBatch:
-    """Many meshes' EvalStencils in one persistent launch (no counterpart in the reference;
+    """Many meshes' EvalStencils in a few persistent launches (no counterpart in the reference;
     the per-mesh equivalent is one EvalStencilsTable call per job).
 
     ``jobs`` is a sequence of ``(table, src, srcDesc, dst, dstDesc)``: a
