@@ -129,10 +129,10 @@ typedef struct GB300StencilTable GB300StencilTable;
  * same source rows together.  The Get*Buffer arrays hold that layout.  The table also keeps a
  * second, evaluation-only copy built on the device (32-stencil slices stored entry-major, in
  * locality order), which GB300StencilTableEval reads; it takes about as much device memory
- * as the Get*Buffer arrays.  A table of one weight array with 65,536 stencils or more keeps a third
+ * as the Get*Buffer arrays.  A table of one weight array with 262,144 stencils or more keeps a third
  * one, in which stencils with the same control indices are evaluated together (a quarter to two
- * thirds of the arrays' size), for large tables and for batches; without memory for it the
- * table does without. */
+ * thirds of the arrays' size); one with 65,536 or more gets it from the first batch that it is part
+ * of.  Without memory for it the table does without. */
 GB300StencilTable *GB300StencilTableCreate(int numStencils, int64_t nnz, const int *sizes,
                                            const int *offsets, const int *indices,
                                            const float *weights, const float *duWeights,

@@ -10,6 +10,7 @@
 #include "units.h"
 
 #include <algorithm>
+#include <mutex>
 #include <new>
 #include <thread>
 #include <vector>
@@ -103,22 +104,30 @@ struct GB300StencilTable {
     // Sliced evaluation layout (sell.h): sz, sliceSlot, idx, w x 6, outRow
     gb300::SellTable sell;
     void *sbuf[10] = {nullptr};
-    // Unit layout (units.h) of a large table with one weight array: slice, blob
+    // Unit layout (units.h) of a large table with one weight array: slice, blob.  Built with the table
+    // if single calls may take it, which read it without a lock, else by the first batch that may
     gb300::UnitTable unit;
     void *ubuf[2] = {nullptr};
+    std::mutex unitLock;
+    bool unitTried = false;
+    int build_unit(const void *const *b, cudaStream_t s, const char *who) {
+        bool one = b[3] && numStencils >= gb300::kUnitTable;
+        for (int k = 4; k < 9; ++k) one = one && !b[k];
+        const int u = one ? gb300::build_units(numStencils, (const int *)b[0], (const int *)b[1],
+                                               (const int *)b[2], (const float *)b[3], s, unit, ubuf,
+                                               who)
+                          : GB300_OK;
+        if (u == GB300_ERR_OUT_OF_MEMORY) cudaGetLastError();  // the table does without
+        unitTried = u == GB300_OK || u == GB300_ERR_UNSUPPORTED;
+        return u == GB300_ERR_CUDA ? u : GB300_OK;
+    }
     int build_layouts(const void *const *b, cudaStream_t s, const char *who) {
         const int *sizes = (const int *)b[0], *offsets = (const int *)b[1];
         const int *indices = (const int *)b[2];
         const int r = gb300::build_sell(numStencils, sizes, offsets, indices,
                                         (const float *const *)b + 3, s, sell, sbuf, who);
         if (r != GB300_OK) return r == GB300_ERR_UNSUPPORTED ? GB300_OK : r;
-        bool one = b[3] && numStencils >= gb300::kUnitTable;
-        for (int k = 4; k < 9; ++k) one = one && !b[k];
-        if (!one) return GB300_OK;
-        const int u = gb300::build_units(numStencils, sizes, offsets, indices,
-                                         (const float *)b[3], s, unit, ubuf, who);
-        if (u == GB300_ERR_OUT_OF_MEMORY) cudaGetLastError();  // the table does without
-        return u == GB300_ERR_CUDA ? u : GB300_OK;
+        return numStencils >= gb300::kUnitCall ? build_unit(b, s, who) : GB300_OK;
     }
     ~GB300StencilTable() {
         for (auto &p : buf) release(p);
@@ -263,7 +272,13 @@ int stencil_table_num_control(const GB300StencilTable *t) { return t ? t->numCon
 }  // namespace batch
 
 const SellTable *stencil_table_sell(const GB300StencilTable *t) { return t ? &t->sell : nullptr; }
-const UnitTable *stencil_table_units(const GB300StencilTable *t) { return t ? &t->unit : nullptr; }
+int stencil_table_units(GB300StencilTable *t, cudaStream_t s, const char *who, const UnitTable **out) {
+    std::lock_guard<std::mutex> lock(t->unitLock);
+    const bool later = t->numStencils >= kUnitTable && t->numStencils < kUnitCall && !t->unitTried;
+    const int r = later ? t->build_unit(t->buf, s, who) : GB300_OK;
+    *out = &t->unit;
+    return r;
+}
 
 GB300StencilTable *adopt_stencil_table(int numStencils, int64_t nnz, int numControl,
                                        void *const buf[9], cudaStream_t s, const char *who) {
@@ -353,7 +368,7 @@ int table_eval(const GB300StencilTable *t, const float *src, float *const *dIn, 
                         "weights",
                         k);
     }
-    if (t->unit.numStencils > 0 && d[0] && src && units_take(src, srcStride)) {
+    if (t->numStencils >= kUnitCall && d[0] && src && units_take(src, srcStride)) {
         const UnitRows rows = units_rows(t->unit, d[0], st[0], length,
                                          (long long)t->numStencils * st[0] * 4, false);
         if (rows != kUnitNone)

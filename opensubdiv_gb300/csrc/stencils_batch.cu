@@ -1052,7 +1052,6 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
     std::vector<int> rows;
     std::vector<const UnitTable *> units;
     for (int i : order) {
-        units.push_back(stencil_table_units(tables[i]));
         b->jobs.push_back(jobs[i]);
         b->mean.push_back(mean[i]);
         rows.push_back(stencil_table_num_control(tables[i]));
@@ -1062,6 +1061,17 @@ GB300StencilBatch *GB300StencilBatchCreate(int numJobs, GB300StencilTable *const
     for (const Job &j : b->jobs) b->sliced = b->sliced && j.slSz;
     if (!b->sliced)
         for (Job &j : b->jobs) j.slSz = nullptr;
+    static const UnitTable none;
+    long long large = 0;  // stencils of the jobs that the unit layout may take
+    for (const Job &j : jobs) large += j.numStencils >= kUnitTable ? j.numStencils : 0;
+    for (int i : order) {
+        units.push_back(&none);
+        if (b->sliced && large >= 2 * kUnitTable &&
+            stencil_table_units(tables[i], s, "GB300StencilBatchCreate", &units.back()) != GB300_OK) {
+            delete b;
+            return nullptr;
+        }
+    }
     if (setup_padding(b, rows, s) != GB300_OK) {
         delete b;
         return nullptr;

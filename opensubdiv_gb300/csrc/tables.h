@@ -15,8 +15,10 @@ struct UnitTable;
 // The table's sliced evaluation layout (numSlices 0 when it has none).
 const SellTable *stencil_table_sell(const GB300StencilTable *table);
 
-// The table's unit layout (numSlices 0 when it has none).
-const UnitTable *stencil_table_units(const GB300StencilTable *table);
+// The table's unit layout (numSlices 0 when it has none), for a batch: of a table below the size from
+// which single calls take it, it is built here, once (on stream `s`, which is waited for).
+int stencil_table_units(GB300StencilTable *table, cudaStream_t s, const char *who,
+                        const UnitTable **out);
 
 // Wraps device buffers (sizes, offsets, indices, w, du, dv, duu, duv, dvv; unused = null, all
 // allocated with cudaMalloc) in a table object that owns them, and builds its

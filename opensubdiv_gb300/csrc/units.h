@@ -39,8 +39,9 @@ struct UnitTable {
     int numStencils = 0;
 };
 
-// Tables from kUnitTable stencils on get the layout beside the sliced one.  A single call takes it from
-// kUnitCall on; below, there are too few slices for the SMs' warps (8-wide level-3 rows, against the
+// Tables from kUnitTable stencils on may have the layout beside the sliced one: from kUnitCall on they get
+// it when they are made, smaller ones in the first batch that may take it (a table of 69 k stencils was
+// made in 2.6 ms before the layout, 3.1 with it).  A single call takes it from kUnitCall on; below, there are too few slices for the SMs' warps (8-wide level-3 rows, against the
 // sliced layout: 131 k stencils 10.3 and 10.3 us, 295 k 12.3 and 14.7 us, 524 k 14.8 and 20.7 us, 1.2 M
 // 29.1 and 39.0 us).  A batch's jobs fill the SMs together: it takes the layout for all of them when
 // they have 2 * kUnitTable stencils between them (one job of 75 k stencils, 3- and 12-wide: 13.8 and
